@@ -25,6 +25,7 @@
 #include "../../include/gmk.h"
 #include "enum_core.cuh"
 #include "enum_warp.cuh"
+#include "enum_dense.cuh"
 #include "mlp.cuh"
 
 namespace {
@@ -160,6 +161,9 @@ constexpr uint32_t kDefaultWarpArena = 1u << 18;
 #define GMK_DONATE_MIN 16
 #endif
 constexpr uint32_t kDefaultDonateMin = GMK_DONATE_MIN;
+// The same for the small graphs' search, whose nodes cost a tenth of a
+// list-based one and whose records are one state.
+constexpr uint32_t kDenseDonateMin = 1;
 
 // One graph of a launch.  A launch enumerates one graph (gmk_enumerate) or a
 // batch of graphs (gmk_enumerate_batch); each has its own k, chunking, root
@@ -434,6 +438,239 @@ enumerate_warp_kernel(const __grid_constant__ WarpArgs a) {
     flush(t, o);
 }
 
+// Small graphs (at most 32 N vertices a side): the bit-mask search of
+// enum_dense.cuh, one task per warp at a time, states shared inside the launch.
+struct DenseArgs {
+    GraphTask single;                  // the graph of a one-graph launch (kernel parameter)
+    const GraphTask* graphs;           // the graphs of a batch launch
+    uint32_t n_graphs;
+    Counters* ctr;                     // stop / error / watchdog origin of the launch
+    RoundCounters* rc;
+    uint32_t* spill;
+    unsigned long long queue_len;
+    const TaskEntry* tasks;            // planned root tasks (pad = graph), or null
+    gmk::dense::Share share;           // share.rec null: no sharing
+    unsigned long long limit;          // one graph: the run's result limit
+    unsigned long long watchdog_ns;
+};
+
+// Resident one-warp blocks per SM: the register allocation targets these.
+// 64 registers hold the N = 1 search without spills; N = 2 and 4 keep 4 and 16
+// mask words a side per lane.
+constexpr int dense_blocks(int n) { return n == 1 ? 32 : n == 2 ? 24 : n == 3 ? 18 : 16; }
+
+template <int N, bool kBatch>
+__global__ void __launch_bounds__(32, dense_blocks(N))
+enumerate_dense_kernel(const __grid_constant__ DenseArgs a) {
+    using namespace gmk::dense;
+    __shared__ Shared<N> sh;
+    Ctx<N> t;
+    t.lane = threadIdx.x;
+    t.sh = &sh;
+    t.spill = a.spill + (unsigned long long)blockIdx.x * spill_words<N>();
+    t.nfound = t.sp = t.bottom = 0;
+    t.cnt = t.hsum = t.hxor = t.nodes = t.work = 0;
+    const uint32_t lane = t.lane;
+    const bool share = a.share.rec != nullptr;
+    unsigned long long deadline = 0;
+    if (a.watchdog_ns) {
+        unsigned long long t0 = 0;
+        if (lane == 0) {
+            const unsigned long long now = gmk::now_ns();
+            const unsigned long long old = atomicCAS(&a.ctr->t0_ns, 0ull, now);
+            t0 = old ? old : now;
+        }
+        deadline = bcast(t0) + a.watchdog_ns;
+    }
+    uint32_t gid = 0xFFFFFFFFu;
+    unsigned long long limit = a.limit;
+    Counters* ctr = nullptr;
+    // results and nodes of the current graph so far to its counters
+    auto flush = [&]() {
+        if (t.nfound) flush_found<N>(t);
+        const unsigned long long work = gmk::warp::warp_sum64(t.work);
+        if (lane == 0 && ctr) {
+            if (t.cnt) {
+                const unsigned long long before = atomicAdd(&ctr->count, t.cnt);
+                atomicAdd(&ctr->hash_sum, t.hsum);
+                atomicXor(&ctr->hash_xor, t.hxor);
+                if (limit && before + t.cnt >= limit) atomicExch(kBatch ? &ctr->stop : &a.ctr->stop, 1);
+            }
+            if (t.nodes) atomicAdd(&ctr->nodes, t.nodes);
+            if (work) atomicAdd(&ctr->work, work);
+        }
+        t.cnt = t.hsum = t.hxor = t.nodes = t.work = 0;
+    };
+    for (;;) {
+        unsigned long long j = ~0ull;
+        int stop = 0;
+        if (lane == 0) {
+            stop = gmk::load_flag(&a.ctr->stop);
+            if (!stop) j = atomicAdd(&a.rc->next_task, 1ull);
+        }
+        stop = bcast(stop);
+        j = bcast(j);
+        if (stop) break;
+        State<N> s;
+        uint32_t next_gid = 0, root = 0, y = 0, y_end = 0;
+        bool have = true;
+        if (j >= a.queue_len) {
+            // take a ticket and wait for its slot's record, or for the end of
+            // the launch's work (no task outstanding)
+            if (!share) break;
+            int quit = 0;
+            unsigned long long ticket = 0;
+            if (lane == 0) {
+                ticket = atomicAdd(a.share.claim, 1ull);
+                const volatile uint32_t* slot = a.share.rec + ticket * kRecordWords;
+                unsigned long long seen = ~0ull, t_seen = gmk::now_ns();
+                unsigned sleep_ns = 32;
+                for (uint32_t spin = 0;; ++spin) {
+                    if (ticket < a.share.slots && *slot == a.share.launch) break;
+                    if ((spin & 7u) == 7u) {
+                        if (gmk::load_flag(&a.ctr->stop)) { quit = 1; break; }
+                        const unsigned long long out = *(volatile unsigned long long*)a.share.outstanding;
+                        if (out + a.queue_len == 0) { quit = 1; break; }
+                        // safety net: the work left must change within the limit
+                        const unsigned long long sig = out + 0x9E3779B97F4A7C15ull *
+                                                       *(volatile unsigned long long*)a.share.tail;
+                        const unsigned long long now = gmk::now_ns();
+                        if (sig != seen) {
+                            seen = sig;
+                            t_seen = now;
+                        } else if (now - t_seen > kIdleLimitNs) {
+                            atomicCAS(&a.ctr->error, 0, gmk::TASK_E_TIMEOUT);
+                            atomicExch(&a.ctr->stop, 1);
+                            quit = 1;
+                            break;
+                        }
+                    }
+                    __nanosleep(sleep_ns);
+                    sleep_ns = sleep_ns < GMK_IDLE_SLEEP_MAX ? sleep_ns * 2 : sleep_ns;
+                }
+                __threadfence();
+            }
+            quit = bcast(quit);
+            if (quit) break;
+            ticket = bcast(ticket);
+            // (written moments ago by a warp on another SM: L2-coherent loads)
+            const uint32_t* r = a.share.rec + ticket * kRecordWords;
+            next_gid = kBatch ? __ldcg(r + 1) : 0u;
+            #pragma unroll
+            for (int w = 0; w < N; ++w) {
+                s.iu[w] = __ldcg(r + kHeader + w); s.iv[w] = __ldcg(r + kHeader + N + w);
+                s.cu[w] = __ldcg(r + kHeader + 2 * N + w); s.cv[w] = __ldcg(r + kHeader + 3 * N + w);
+            }
+        } else {
+            if (lane == 0) atomicAdd(&a.rc->tasks_done, 1ull);
+            TaskEntry e{0, 0, 0, 0};
+            if (a.tasks) {
+                e = a.tasks[j];
+                next_gid = kBatch ? e.pad : 0u;
+            } else if (kBatch) {
+                uint32_t hi = a.n_graphs;
+                while (hi - next_gid > 1) {
+                    const uint32_t mid = (next_gid + hi) >> 1;
+                    if (a.graphs[mid].task_begin <= j) next_gid = mid; else hi = mid;
+                }
+            }
+            const GraphTask& G = kBatch ? a.graphs[next_gid] : a.single;
+            const uint32_t nl = G.g.nl, n = G.g.n;
+            if (!a.tasks) {
+                const unsigned long long local = j - G.task_begin;
+                e.root = G.root_base + (uint32_t)(local % G.n_roots);
+                e.first = nl + (uint32_t)(local / G.n_roots) * G.chunk;
+                e.last = n - e.first > G.chunk ? e.first + G.chunk : n;
+            }
+            root = e.root;
+            y = e.first - nl;
+            y_end = e.last - nl;
+            have = e.first <= nl && e.last >= n;   // the whole root: one state
+            if (have) y = y_end;
+            #pragma unroll
+            for (int w = 0; w < N; ++w) {
+                s.iu[w] = root >> 5 == (uint32_t)w ? 1u << (root & 31u) : 0u;
+                s.iv[w] = 0;
+                s.cu[w] = low_bits(nl, w) & ~low_bits(root + 1, w);
+                s.cv[w] = low_bits(n - nl, w);
+            }
+        }
+        const GraphTask& G = kBatch ? a.graphs[next_gid] : a.single;
+        if (next_gid != gid) {
+            flush();
+            gid = next_gid;
+            ctr = G.ctr;
+            t.k = G.k;
+            if (kBatch) limit = G.limit;
+            load_graph<N>(t, G.g);
+        }
+        // (a state's root is its smallest included U vertex)
+        #pragma unroll
+        for (int w = N - 1; w >= 0; --w)
+            if (s.iu[w]) root = 32 * w + __ffs(s.iu[w]) - 1;
+        t.sp = t.bottom = 0;
+        uint32_t polls = 0;
+        unsigned long long nodes = 0;
+        bool quit = kBatch && gmk::load_flag(&ctr->stop);   // a capped graph's tasks end at once
+        quit = __any_sync(gmk::warp::kFull, quit);
+        while (!quit) {
+            if (!have) {
+                if (y >= y_end) break;
+                // the next first-level child: after x, after y
+                const uint32_t nl = G.g.nl, nv = G.g.n - nl;
+                #pragma unroll
+                for (int w = 0; w < N; ++w) {
+                    s.iu[w] = root >> 5 == (uint32_t)w ? 1u << (root & 31u) : 0u;
+                    s.iv[w] = y >> 5 == (uint32_t)w ? 1u << (y & 31u) : 0u;
+                    s.cu[w] = low_bits(nl, w) & ~low_bits(root + 1, w);
+                    s.cv[w] = low_bits(nv, w) & ~low_bits(y + 1, w);
+                }
+                refit<N>(t, s);
+                ++y;
+                have = true;
+            }
+            if (++polls == poll_nodes<N>()) {
+                polls = 0;
+                int late = 0, want = 0, done = 0;
+                if (lane == 0) {
+                    done = gmk::load_flag(&a.ctr->stop) || (kBatch && gmk::load_flag(&ctr->stop));
+                    late = deadline && gmk::now_ns() > deadline;
+                    if (share && nodes >= a.share.min_nodes && t.sp != t.bottom && !gmk::load_flag(a.share.full)) {
+                        const long long w = (long long)(*(volatile const unsigned long long*)a.share.claim -
+                                                        *(volatile const unsigned long long*)a.share.tail);
+                        want = w > 0 ? (int)(w < 32 ? w : 32) : 0;
+                    }
+                }
+                done = bcast(done); late = bcast(late); want = bcast(want);
+                if (late && lane == 0) {
+                    atomicCAS(&a.ctr->error, 0, gmk::TASK_E_TIMEOUT);
+                    atomicExch(&a.ctr->stop, 1);
+                }
+                if (done || late) { quit = true; break; }
+                if (want) donate<N>(t, a.share, gid, (uint32_t)want);
+                if (limit && t.cnt >= gmk::kFlushBatch) flush();
+            }
+            ++nodes;
+            if (!node<N>(t, s)) {
+                if (t.sp == t.bottom) {
+                    have = false;
+                } else {
+                    --t.sp;
+                    __syncwarp();
+                    read_state<N>(stack_at<N>(t, t.sp), s);
+                    __syncwarp();
+                }
+            }
+        }
+        t.nodes += nodes;
+        if (lane == 0) {
+            if (G.root_nodes) atomicAdd(G.root_nodes + root, nodes);
+            if (share) atomicAdd(a.share.outstanding, ~0ull);   // this task is finished
+        }
+    }
+    flush();
+}
+
 // CSR check on the device: thread i checks vertex i (offsets non-decreasing
 // and within adj) and adjacency entry i (inside its row, ascending, an id of
 // the other side), so a hub's row is spread over many threads.  It also folds
@@ -558,6 +795,18 @@ struct Workspace {
     unsigned long long* d_dq_idx = nullptr;
     size_t dq_idx_bytes = 0;
     unsigned long long dq_dirty = 0;
+    // small graphs' search: stack spill, records of shared states (each valid for
+    // the launch whose number it carries), counters of a launch and their pinned
+    // copy on the host
+    uint32_t* d_spill = nullptr;
+    size_t spill_bytes = 0;
+    uint32_t* d_states = nullptr;
+    size_t states_bytes = 0;
+    uint32_t dense_launch = 0;
+    void* d_dense = nullptr;
+    size_t dense_bytes = 0;
+    void* h_dense = nullptr;
+    size_t h_dense_bytes = 0;
     // pinned staging of the planned task table: the call does not wait for its
     // copy; the next call waits on tasks_ev before it refills the buffer
     void* h_tasks = nullptr;
@@ -571,6 +820,7 @@ Workspace g_ws[kMaxDevices];
 struct DeviceInfo {
     bool ready = false;
     int sms = 0, per_sm_warp = 0, per_sm_batch = 0, per_sm_thread = 0;
+    int per_sm_dense[5][2] = {};   // [N = 1..4][one graph, batch]
 };
 DeviceInfo g_dev[kMaxDevices];
 
@@ -1014,6 +1264,288 @@ struct GraphJob {
     uint64_t* root_nodes;         // optional host log
 };
 
+// Does the run take its tasks from a plan (by cost, for a shard, or given)?
+// (a plain run given costs keeps one task per root and no splitting, but
+// starts the largest predicted roots first: the static schedule with the
+// learned order)
+bool is_planned(const std::vector<GraphJob>& jobs, const gmk_opts* opts) {
+    return opts->schedule == GMK_SCHEDULE_ORDERED || opts->nshards > 1 || opts->tasks ||
+           (opts->schedule == GMK_SCHEDULE_PLAIN && jobs[0].task_cost);
+}
+
+// The planned tasks of a run for `workers` workers, at most max_chunks a root.
+int plan_jobs(std::vector<GraphJob>& jobs, const gmk_opts* opts, uint64_t workers,
+              uint32_t max_chunks, std::vector<gmk_task>& plan) {
+    int rc;
+    const size_t ng = jobs.size();
+    const uint32_t nsh = opts->nshards > 1 ? opts->nshards : 1u;
+    const uint32_t sh = nsh > 1 ? opts->shard : 0u;
+    const uint32_t tasks_per = opts->tasks_per_worker ? opts->tasks_per_worker : 8u;
+    if (opts->tasks) {
+        // the caller's list, as given (checked by gmk_enumerate)
+        plan.assign(opts->tasks, opts->tasks + opts->n_tasks);
+        for (gmk_task& t : plan) t.graph = 0;
+        return GMK_OK;
+    }
+    std::vector<const float*> costs(ng);
+    std::vector<std::vector<uint32_t>> roots(ng);
+    double total = 0;
+    for (size_t i = 0; i < ng; ++i) {
+        const GraphJob& j = jobs[i];
+        costs[i] = j.task_cost;
+        if (!costs[i] && (rc = proxy_costs(j.g, &costs[i]))) return rc;
+        roots[i] = select_roots(j.g->nl, costs[i], j.root_begin, j.root_end);
+        for (const uint32_t r : roots[i]) total += std::max<double>(costs[i][r], 0.0);
+    }
+    const double unit = total / (double)std::max<uint64_t>(1, (uint64_t)tasks_per * workers);
+    for (size_t i = 0; i < ng; ++i)
+        chunk_roots(jobs[i].g->nl, jobs[i].g->n, roots[i], costs[i], unit, max_chunks,
+                    (uint32_t)i, plan);
+    order_and_shard(plan, nsh, sh, ng == 1);
+    // Under a result limit (the run's, or a batch graph's cap) balance does
+    // not matter (every warp stays busy until the limit); how many search
+    // nodes the first `limit` results cost does, and that depends on the
+    // order.  The model predicts node counts, not result density: largest
+    // first took 4-36x longer to the limit than id order, cheapest first
+    // 1.1-1.25x less at k = 2 but 1.4-7x more at k = 1 (cl500k: 632 M
+    // nodes for 10^8 results against 60 M).  So capped runs keep each
+    // graph's roots in id order (the plain schedule's), chunks as planned.
+    bool capped = opts->result_limit != 0;
+    for (const GraphJob& j : jobs) capped |= j.limit != 0;
+    if (capped) {
+        std::sort(plan.begin(), plan.end(), [](const gmk_task& a, const gmk_task& b) {
+            if (a.graph != b.graph) return a.graph < b.graph;
+            return a.root != b.root ? a.root < b.root : a.first < b.first;
+        });
+    }
+    return GMK_OK;
+}
+
+// Copies a plan to the graph's device task table through the pinned staging
+// buffer (the call does not wait for the copy).
+int upload_plan(Workspace& ws, gmk_graph* g0, const std::vector<gmk_task>& plan) {
+    if (plan.empty()) return GMK_OK;
+    const size_t bytes = sizeof(TaskEntry) * plan.size();
+    if (!ws.tasks_ev) CK(cudaEventCreateWithFlags(&ws.tasks_ev, cudaEventDisableTiming));
+    CK(cudaEventSynchronize(ws.tasks_ev));   // the last call's copy has left the buffer
+    if (ws.h_tasks_bytes < bytes) {
+        if (ws.h_tasks) CK(cudaFreeHost(ws.h_tasks));
+        ws.h_tasks = nullptr;
+        ws.h_tasks_bytes = 0;
+        CK(cudaHostAlloc(&ws.h_tasks, bytes, cudaHostAllocDefault));
+        ws.h_tasks_bytes = bytes;
+    }
+    TaskEntry* tab = static_cast<TaskEntry*>(ws.h_tasks);
+    for (size_t i = 0; i < plan.size(); ++i)
+        tab[i] = TaskEntry{plan[i].root, plan[i].first, plan[i].last, plan[i].graph};
+    if (int rc = pool_grow(g0->device, (void**)&g0->d_tasks, &g0->tasks_bytes, bytes)) return rc;
+    CK(cudaMemcpyAsync(g0->d_tasks, tab, bytes, cudaMemcpyHostToDevice, g0->stream));
+    CK(cudaEventRecord(ws.tasks_ev, g0->stream));
+    return GMK_OK;
+}
+
+// The status of a kernel's error code.
+int task_status(int error) {
+    switch (error) {
+        case gmk::TASK_OK: return GMK_OK;
+        case gmk::TASK_E_ARENA: return GMK_E_ARENA;
+        case gmk::TASK_E_SMAX: return GMK_E_SMAX;
+        case gmk::TASK_E_TIMEOUT: return GMK_E_TIMEOUT;
+        case gmk::TASK_E_OUTBUF: return GMK_E_OUTBUF;
+        case gmk::TASK_E_RECORD:
+            g_cuda_err = "a split or donated task record failed its checks (internal error)";
+            return GMK_E_CUDA;
+        default: return GMK_E_CUDA;
+    }
+}
+
+// Vertices a side that the bit-mask search of small graphs takes (its N = 4).
+constexpr uint32_t kDenseSide = 128;
+
+// First-level children per task there.  One state per root starts with as many
+// tasks as roots, and the rest spreads state by state: 77 x 77, k = 2 took 21.4 ms
+// that way, 14.2 with 1 or 2 children a task (100 x 99, k = 1: 1.12 with 1, 1.05
+// with 2).
+constexpr uint32_t kDenseChunk = 2;
+
+// Mask words a side (1 to 4) when this run goes to the bit-mask search of
+// small graphs, else 0: count-only warp-engine runs in one launch over graphs
+// of at most kDenseSide vertices a side (at 128 x 128 it is still 3.7x faster
+// than the list-based search, at four words a mask; eight would not leave a
+// lane registers for them).  Runs that bound the list-based
+// search's memory or rules (arena_words, max_members, pair_limit,
+// bits_min_list) or that ask for splitting into launches (no_sharing) keep it,
+// and so do records.
+int dense_words(const std::vector<GraphJob>& jobs, const gmk_opts* opts) {
+    if (opts->engine != GMK_ENGINE_WARP || opts->emit || opts->no_sharing || opts->arena_words ||
+        opts->max_members || opts->pair_limit || opts->bits_min_list)
+        return 0;
+    uint32_t side = 0;
+    for (const GraphJob& j : jobs) side = std::max({side, j.g->nl, j.g->n - j.g->nl});
+    if (side > kDenseSide) return 0;
+    return (int)(std::max<uint32_t>(side, 1) + 31) / 32;
+}
+
+// Counters of a small-graph launch, device and host side: one block, so one
+// memset and one copy a call.
+struct DenseCounters {
+    RoundCounters rc;
+    Counters launch;       // stop, error, watchdog origin; the counts of a one-graph run
+    Counters graph[1];     // batches: one per graph
+};
+
+template <int N>
+int dense_occupancy(DeviceInfo& di) {
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&di.per_sm_dense[N][0], enumerate_dense_kernel<N, false>,
+                                                     32, 0));
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&di.per_sm_dense[N][1], enumerate_dense_kernel<N, true>,
+                                                     32, 0));
+    return GMK_OK;
+}
+
+template <int N>
+void launch_dense(const DenseArgs& a, unsigned grid, bool batch, cudaStream_t s) {
+    if (batch) enumerate_dense_kernel<N, true><<<grid, 32, 0, s>>>(a);
+    else enumerate_dense_kernel<N, false><<<grid, 32, 0, s>>>(a);
+}
+
+// run_jobs for small graphs: one launch of the bit-mask search.
+int run_dense(std::vector<GraphJob>& jobs, const gmk_opts* opts, int words, Workspace& ws,
+              const DeviceInfo& di, gmk_stats* outs) {
+    gmk_graph* g0 = jobs[0].g;
+    const size_t ng = jobs.size();
+    const uint64_t resident = (uint64_t)di.sms * std::max(di.per_sm_dense[words][ng > 1], 1);
+    const uint64_t workers = opts->threads ? std::max<uint64_t>(1, ((uint64_t)opts->threads + 31) / 32)
+                                           : resident;
+    int rc;
+    std::vector<gmk_task> plan;
+    const bool planned = is_planned(jobs, opts);
+    const uint32_t max_chunks = opts->schedule == GMK_SCHEDULE_PLAIN ? 1u : 0xFFFFFFFFu;
+    if (planned) {
+        if ((rc = plan_jobs(jobs, opts, workers, max_chunks, plan))) return rc;
+        if ((rc = upload_plan(ws, g0, plan))) return rc;
+    }
+    const size_t ctr_bytes = sizeof(DenseCounters) + (ng > 1 ? (ng - 1) * sizeof(Counters) : 0);
+    if ((rc = grow(&ws.d_dense, &ws.dense_bytes, ctr_bytes))) return rc;
+    if (ws.h_dense_bytes < ctr_bytes) {
+        if (ws.h_dense) CK(cudaFreeHost(ws.h_dense));
+        ws.h_dense = nullptr;
+        ws.h_dense_bytes = 0;
+        CK(cudaHostAlloc(&ws.h_dense, ctr_bytes, cudaHostAllocDefault));
+        ws.h_dense_bytes = ctr_bytes;
+    }
+    DenseCounters* dc = static_cast<DenseCounters*>(ws.d_dense);
+    unsigned long long n_tasks = 0;
+    std::vector<GraphTask> gt(ng);
+    for (size_t i = 0; i < ng; ++i) {
+        const GraphJob& j = jobs[i];
+        gmk_graph* g = j.g;
+        const uint32_t nv = g->n - g->nl;
+        GraphTask& t = gt[i];
+        t.g = gmk::GraphView{g->d_off, g->d_adj, g->n, g->nl};
+        t.eh.slots = g->d_eh;
+        t.eh.bmask = g->eh_bmask;
+        t.k = j.k;
+        t.chunk = opts->schedule == GMK_SCHEDULE_PLAIN ? nv : std::min(opts->chunk ? opts->chunk : kDenseChunk, nv);
+        t.n_roots = j.root_end - j.root_begin;
+        t.root_base = j.root_begin;
+        t.limit = j.limit;
+        t.ctr = ng > 1 ? &dc->graph[i] : &dc->launch;
+        t.root_nodes = nullptr;
+        if (j.root_nodes) {
+            if (!g->d_root_nodes)
+                CK(pool_alloc(g->device, (void**)&g->d_root_nodes, 8ull * std::max<uint32_t>(g->nl, 1)));
+            CK(cudaMemsetAsync(g->d_root_nodes, 0, 8ull * g->nl, g0->stream));
+            t.root_nodes = g->d_root_nodes;
+        }
+        t.task_begin = n_tasks;
+        if (!planned) n_tasks += (unsigned long long)t.n_roots * ((nv + t.chunk - 1) / t.chunk);
+    }
+    if (planned) n_tasks = plan.size();
+    if (ng > 1) {
+        if ((rc = grow((void**)&ws.d_graphs, &ws.graphs_bytes, sizeof(GraphTask) * ng))) return rc;
+        CK(cudaMemcpyAsync(ws.d_graphs, gt.data(), sizeof(GraphTask) * ng, cudaMemcpyHostToDevice,
+                           g0->stream));
+    }
+    const size_t spill = 4ull * (words == 1   ? gmk::dense::spill_words<1>()
+                                 : words == 2 ? gmk::dense::spill_words<2>()
+                                 : words == 3 ? gmk::dense::spill_words<3>()
+                                              : gmk::dense::spill_words<4>());
+    if ((rc = grow((void**)&ws.d_spill, &ws.spill_bytes, std::max<size_t>(256, workers * spill)))) return rc;
+    DenseArgs a;
+    std::memset(&a, 0, sizeof(a));
+    if (opts->schedule != GMK_SCHEDULE_PLAIN) {
+        const uint64_t slots = std::max<uint64_t>(1ull << 16, workers * 128ull);
+        const size_t need = slots * gmk::dense::kRecordWords * 4;
+        const void* had = ws.d_states;
+        if ((rc = grow((void**)&ws.d_states, &ws.states_bytes, need))) return rc;
+        // a record counts when it carries this launch's number; a new buffer,
+        // and one whose numbers are used up, starts cleared
+        if (ws.d_states != had || ++ws.dense_launch == 0) {
+            CK(cudaMemsetAsync(ws.d_states, 0, ws.states_bytes, g0->stream));
+            ws.dense_launch = 1;
+        }
+        a.share.rec = ws.d_states;
+        a.share.slots = (uint32_t)slots;
+        a.share.launch = ws.dense_launch;
+        a.share.tail = &dc->rc.dq_tail;
+        a.share.claim = &dc->rc.dq_claim;
+        a.share.outstanding = &dc->rc.outstanding;
+        a.share.donated = &dc->rc.donated;
+        a.share.full = &dc->rc.dq_full;
+        a.share.min_nodes = opts->donate_min_nodes ? opts->donate_min_nodes : kDenseDonateMin;
+    }
+    a.single = gt[0];
+    a.graphs = static_cast<const GraphTask*>(ws.d_graphs);
+    a.n_graphs = (uint32_t)ng;
+    a.ctr = &dc->launch;
+    a.rc = &dc->rc;
+    a.spill = ws.d_spill;
+    a.queue_len = n_tasks;
+    a.tasks = planned && !plan.empty() ? g0->d_tasks : nullptr;
+    a.limit = ng > 1 ? 0 : opts->result_limit ? opts->result_limit : jobs[0].limit;
+    a.watchdog_ns = (unsigned long long)opts->watchdog_ms * 1000000ull;
+    CK(cudaEventRecord(g0->ev0, g0->stream));
+    CK(cudaMemsetAsync(dc, 0, ctr_bytes, g0->stream));
+    const unsigned grid = (unsigned)workers;
+    if (words == 1) launch_dense<1>(a, grid, ng > 1, g0->stream);
+    else if (words == 2) launch_dense<2>(a, grid, ng > 1, g0->stream);
+    else if (words == 3) launch_dense<3>(a, grid, ng > 1, g0->stream);
+    else launch_dense<4>(a, grid, ng > 1, g0->stream);
+    CK(cudaGetLastError());
+    CK(cudaEventRecord(g0->ev1, g0->stream));
+    CK(cudaMemcpyAsync(ws.h_dense, dc, ctr_bytes, cudaMemcpyDeviceToHost, g0->stream));
+    CK(cudaStreamSynchronize(g0->stream));
+    const DenseCounters* h = static_cast<const DenseCounters*>(ws.h_dense);
+    for (size_t i = 0; i < ng; ++i) {
+        if (!jobs[i].root_nodes) continue;
+        gmk_graph* g = jobs[i].g;
+        std::vector<unsigned long long> rn(g->nl);
+        CK(cudaMemcpy(rn.data(), g->d_root_nodes, 8ull * g->nl, cudaMemcpyDeviceToHost));
+        for (uint32_t v = 0; v < g->nl; ++v) jobs[i].root_nodes[v] += rn[v];
+    }
+    float ms = 0.f;
+    CK(cudaEventElapsedTime(&ms, g0->ev0, g0->ev1));
+    for (size_t i = 0; i < ng; ++i) {
+        const Counters& hc = ng > 1 ? h->graph[i] : h->launch;
+        const unsigned long long cap = ng > 1 ? jobs[i].limit : a.limit;
+        gmk_stats* out = outs + i;
+        out->count = cap ? std::min<unsigned long long>(hc.count, cap) : hc.count;
+        out->hash_sum = hc.hash_sum;
+        out->hash_xor = hc.hash_xor;
+        out->nodes = hc.nodes;
+        out->algo_bytes = 4ull * hc.work;
+        out->tasks = n_tasks;
+        out->tasks_done = std::min<unsigned long long>(h->rc.tasks_done, n_tasks);
+        out->kernel_ms = ms;
+        out->truncated = cap && hc.count >= cap;
+        out->threads = (uint32_t)(workers * 32);
+        out->rounds = 1;
+        out->donations = h->rc.donated;
+    }
+    return task_status(h->launch.error);
+}
+
 // Enumerates the jobs' graphs (all on one device) in one run of launches and
 // fills outs[i] per graph.  The single-graph call and the batch call share it;
 // a batch needs the warp engine, no records and no sharding (checked by the
@@ -1035,9 +1567,14 @@ int run_jobs(std::vector<GraphJob>& jobs, const gmk_opts* opts, gmk_sink sink, v
             &di.per_sm_batch, enumerate_warp_kernel<true, false, false>, kWBlock, 0));
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&di.per_sm_thread, enumerate_kernel,
                                                          kBlock, 0));
+        if (int rc = dense_occupancy<1>(di)) return rc;
+        if (int rc = dense_occupancy<2>(di)) return rc;
+        if (int rc = dense_occupancy<3>(di)) return rc;
+        if (int rc = dense_occupancy<4>(di)) return rc;
         di.sms = sms;
         di.ready = true;
     }
+    if (const int words = dense_words(jobs, opts)) return run_dense(jobs, opts, words, ws, di, outs);
     // resident blocks per SM of the instantiation this run launches
     const int per_sm = std::max(!warp ? di.per_sm_thread : jobs.size() > 1 ? di.per_sm_batch : di.per_sm_warp, 1);
     const int block = warp ? kWBlock : kBlock;
@@ -1098,53 +1635,11 @@ int run_jobs(std::vector<GraphJob>& jobs, const gmk_opts* opts, gmk_sink sink, v
     const size_t ng = jobs.size();
     std::vector<GraphTask> gt(ng);
     std::vector<uint32_t> chunks(ng), cprs(ng);
-    const uint32_t nsh = opts->nshards > 1 ? opts->nshards : 1u;
-    const uint32_t sh = nsh > 1 ? opts->shard : 0u;
     const uint32_t tasks_per = opts->tasks_per_worker ? opts->tasks_per_worker : 8u;
-    // (a plain run given costs keeps one task per root and no splitting, but
-    // starts the largest predicted roots first: the static schedule with the
-    // learned order)
-    const bool planned = opts->schedule == GMK_SCHEDULE_ORDERED || nsh > 1 || opts->tasks ||
-                         (opts->schedule == GMK_SCHEDULE_PLAIN && jobs[0].task_cost);
+    const bool planned = is_planned(jobs, opts);
     std::vector<gmk_task> plan;
-    if (opts->tasks) {
-        // the caller's list, as given (checked by gmk_enumerate)
-        plan.assign(opts->tasks, opts->tasks + opts->n_tasks);
-        for (gmk_task& t : plan) t.graph = 0;
-    } else if (planned) {
-        std::vector<const float*> costs(ng);
-        std::vector<std::vector<uint32_t>> roots(ng);
-        double total = 0;
-        for (size_t i = 0; i < ng; ++i) {
-            const GraphJob& j = jobs[i];
-            costs[i] = j.task_cost;
-            if (!costs[i] && (rc = proxy_costs(j.g, &costs[i]))) return rc;
-            roots[i] = select_roots(j.g->nl, costs[i], j.root_begin, j.root_end);
-            for (const uint32_t r : roots[i]) total += std::max<double>(costs[i][r], 0.0);
-        }
-        const uint32_t max_chunks = opts->schedule == GMK_SCHEDULE_PLAIN ? 1u : 0xFFFFFFFFu;
-        const double unit = total / (double)std::max<uint64_t>(1, (uint64_t)tasks_per * workers);
-        for (size_t i = 0; i < ng; ++i)
-            chunk_roots(jobs[i].g->nl, jobs[i].g->n, roots[i], costs[i], unit, max_chunks,
-                        (uint32_t)i, plan);
-        order_and_shard(plan, nsh, sh, ng == 1);
-        // Under a result limit (the run's, or a batch graph's cap) balance does
-        // not matter (every warp stays busy until the limit); how many search
-        // nodes the first `limit` results cost does, and that depends on the
-        // order.  The model predicts node counts, not result density: largest
-        // first took 4-36x longer to the limit than id order, cheapest first
-        // 1.1-1.25x less at k = 2 but 1.4-7x more at k = 1 (cl500k: 632 M
-        // nodes for 10^8 results against 60 M).  So capped runs keep each
-        // graph's roots in id order (the plain schedule's), chunks as planned.
-        bool capped = opts->result_limit != 0;
-        for (const GraphJob& j : jobs) capped |= j.limit != 0;
-        if (capped) {
-            std::sort(plan.begin(), plan.end(), [](const gmk_task& a, const gmk_task& b) {
-                if (a.graph != b.graph) return a.graph < b.graph;
-                return a.root != b.root ? a.root < b.root : a.first < b.first;
-            });
-        }
-    }
+    const uint32_t max_chunks = opts->schedule == GMK_SCHEDULE_PLAIN ? 1u : 0xFFFFFFFFu;
+    if (planned && (rc = plan_jobs(jobs, opts, workers, max_chunks, plan))) return rc;
     unsigned long long n_tasks = 0;
     for (size_t i = 0; i < ng; ++i) {
         const GraphJob& j = jobs[i];
@@ -1189,25 +1684,8 @@ int run_jobs(std::vector<GraphJob>& jobs, const gmk_opts* opts, gmk_sink sink, v
     const TaskEntry* d_tasks = nullptr;
     if (planned) {
         n_tasks = plan.size();
-        if (!plan.empty()) {
-            const size_t bytes = sizeof(TaskEntry) * plan.size();
-            if (!ws.tasks_ev) CK(cudaEventCreateWithFlags(&ws.tasks_ev, cudaEventDisableTiming));
-            CK(cudaEventSynchronize(ws.tasks_ev));   // the last call's copy has left the buffer
-            if (ws.h_tasks_bytes < bytes) {
-                if (ws.h_tasks) CK(cudaFreeHost(ws.h_tasks));
-                ws.h_tasks = nullptr;
-                ws.h_tasks_bytes = 0;
-                CK(cudaHostAlloc(&ws.h_tasks, bytes, cudaHostAllocDefault));
-                ws.h_tasks_bytes = bytes;
-            }
-            TaskEntry* tab = static_cast<TaskEntry*>(ws.h_tasks);
-            for (size_t i = 0; i < plan.size(); ++i)
-                tab[i] = TaskEntry{plan[i].root, plan[i].first, plan[i].last, plan[i].graph};
-            if ((rc = pool_grow(g0->device, (void**)&g0->d_tasks, &g0->tasks_bytes, bytes))) return rc;
-            CK(cudaMemcpyAsync(g0->d_tasks, tab, bytes, cudaMemcpyHostToDevice, g0->stream));
-            CK(cudaEventRecord(ws.tasks_ev, g0->stream));
-            d_tasks = g0->d_tasks;
-        }
+        if ((rc = upload_plan(ws, g0, plan))) return rc;
+        if (!plan.empty()) d_tasks = g0->d_tasks;
     }
     const unsigned long long my_tasks = n_tasks;
     if ((rc = grow((void**)&ws.d_graphs, &ws.graphs_bytes, sizeof(GraphTask) * ng))) return rc;
@@ -1439,17 +1917,7 @@ int run_jobs(std::vector<GraphJob>& jobs, const gmk_opts* opts, gmk_sink sink, v
         out->rounds = rounds;
         out->donations = donations;
     }
-    switch (h.error) {
-        case gmk::TASK_OK: break;
-        case gmk::TASK_E_ARENA: return GMK_E_ARENA;
-        case gmk::TASK_E_SMAX: return GMK_E_SMAX;
-        case gmk::TASK_E_TIMEOUT: return GMK_E_TIMEOUT;
-        case gmk::TASK_E_OUTBUF: return GMK_E_OUTBUF;
-        case gmk::TASK_E_RECORD:
-            g_cuda_err = "a split or donated task record failed its checks (internal error)";
-            return GMK_E_CUDA;
-        default: return GMK_E_CUDA;
-    }
+    if (int st = task_status(h.error)) return st;
     if (warp) return warp_emit_rc;
     if (opts->emit) {
         if (h.out_pos > out_words) return GMK_E_OUTBUF;
