@@ -152,7 +152,8 @@ struct Outputs {
     unsigned long long* out_pos;
     unsigned long long out_cap;     // words
     unsigned long long deadline_ns; // 0 = none; compared with the device's global timer
-    unsigned long long* out_fail;   // warp engine: lowest record position that found no room
+    unsigned long long* out_fail;   // warp engine: complement of the lowest record position that
+                                    //   found no room (0: none)
     int* gstop;                     // warp engine, batches: this graph's limit was reached
                                     //   (null: the limit raises `stop`)
 };

@@ -86,6 +86,7 @@ struct Share {
     unsigned long long* outstanding;  // unfinished tasks - queue_len (mod 2^64)
     unsigned long long* donated;
     int* full;
+    int* done;                        // warp::kDoneFlags flags, as warp::Donation's
     uint32_t min_nodes;
 };
 
@@ -96,6 +97,7 @@ struct Ctx {
     Shared<N>* sh;
     uint32_t* spill;
     uint32_t nfound, sp, bottom;      // stack entries [bottom, sp)
+    uint32_t extra;                   // nodes that subset tests of this task stood for
     unsigned long long cnt, hsum, hxor, nodes, work;
 };
 
@@ -211,10 +213,12 @@ __device__ __forceinline__ void refit(const Ctx<N>& t, State<N>& s) {
     }
 }
 
-// Subsets T of C, one per lane: is I u T (masks lu, lv) a result?
+// Subsets T of C, one per lane: is I u T (masks lu, lv) a result?  *feasible: how
+// many of them are k-biplexes -- the nodes of their set-enumeration tree, which
+// this one node stands for.
 template <int N>
 __device__ __forceinline__ bool subsets(const Ctx<N>& t, const State<N>& s, uint32_t (&lu)[N],
-                                        uint32_t (&lv)[N]) {
+                                        uint32_t (&lv)[N], uint32_t* feasible) {
     const uint32_t lane = t.lane, k = t.k;
     uint32_t j = 0, any_v = 0;
     uint32_t hu[N], hv[N];
@@ -232,7 +236,7 @@ __device__ __forceinline__ bool subsets(const Ctx<N>& t, const State<N>& s, uint
         for (uint32_t y = s.cv[w]; y; y &= y - 1, ++j) lv[w] |= ((lane >> j) & 1u) ? (y & (0u - y)) : 0u;
         any_v |= lv[w];
     }
-    bool alive = (lane >> j) == 0 && any_v != 0;
+    bool alive = (lane >> j) == 0;
     // members: misses, blockers (k or more)
     #pragma unroll
     for (int w = 0; w < N; ++w) {
@@ -259,6 +263,8 @@ __device__ __forceinline__ bool subsets(const Ctx<N>& t, const State<N>& s, uint
             }
         }
     }
+    *feasible = __popc(__ballot_sync(kFull, alive));
+    alive = alive && any_v != 0;
     // nothing left out may join.  A vertex that misses more than k of I, or a
     // vertex of I with k misses in I, joins none of the subsets: only the
     // others are tested subset by subset.
@@ -416,7 +422,9 @@ __device__ __forceinline__ bool node(Ctx<N>& t, State<N>& s) {
             refit<N>(t, s);
             return true;
         }
-        hit = subsets<N>(t, s, lu, lv);
+        uint32_t feasible;
+        hit = subsets<N>(t, s, lu, lv, &feasible);
+        t.extra += feasible - 1;
     }
     const uint32_t who = __ballot_sync(kFull, hit);
     if (hit) {

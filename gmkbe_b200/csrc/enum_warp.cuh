@@ -17,20 +17,20 @@
 //     reference's membership test is binarySearch over sorted rows,
 //     include/gpu_utils.cuh:258-282;
 //   * the search state (frames, lists, S) lives in a per-warp arena, so the
-//     hot part of 4-10k warps' state stays in L2 instead of 150k threads'.
+//     hot part of 2-4k warps' state stays in L2 instead of 150k threads';
+//   * the children of a side that is still global are decided 32 at a time, one
+//     per lane (enum_lanes.cuh), and a node of at most 32 vertices a side is
+//     searched on bit masks (enum_bits.cuh): the lists serve what is larger.
 // Work that outgrows its warp is split: when the task queue of a round is
 // empty, a busy warp writes every frame that still has unexplored children
 // (plus its current node) as separate tasks for the next round.  Together
 // they cover exactly the unexplored part of its search tree.
 //
-// Every search loop carries `#pragma unroll 1`.  The kernel is bound by
-// instruction fetch (the whole search is one kernel, and each warp is at its
-// own point of it): unrolled, the loops and the hash probes inlined into each
-// copy made the count-only kernel 271 KB of machine code; rolled it is 176 KB
-// and 1.07-1.31x faster, the shorter trip counts notwithstanding.  Code size
-// is not the whole story, though: one run_dfs call site for root tasks and
-// records is 1.1-1.5x faster than two inlined copies in the k = 1 kernels,
-// and 1.1x slower in the k >= 2 ones, which keep two.
+// Every search loop carries `#pragma unroll 1`, and the kernel has one call site
+// of everything large: it is bound by instruction fetch (the whole search is one
+// kernel, and each warp is at its own point of it), so code size counts as much
+// as instruction count, and more resident warps can be slower (gmk_capi.cu,
+// kWarpMinBlocks).
 #pragma once
 #include "enum_core.cuh"
 
@@ -47,6 +47,8 @@ constexpr uint32_t FL_ONE_PHASE = 128u;   // frame flag: iterate the current pha
 constexpr uint32_t FL_SHARED0 = 256u;     // frame flags: list 0 / list 1 is a suffix of the
 constexpr uint32_t FL_SHARED1 = 512u;     //   parent's list, read in place (not stored after
                                           //   the frame)
+constexpr uint32_t FL_BUILD = 1024u;      // frame flag: the pending children of its global side
+                                          //   are built (they do not fit lane_blocks)
 constexpr uint32_t kBitsMinList = 64;     // default: shorter lists filter their children by
                                           //   probing (gmk_opts.bits_min_list)
 constexpr uint32_t kBitsMaxZ = 8;         // bitmaps for at most this many members
@@ -96,7 +98,8 @@ __device__ __forceinline__ bool has_edge(const EdgeHash& h, uint32_t a, uint32_t
     const ulonglong2* p = reinterpret_cast<const ulonglong2*>(h.slots + bk * 4);
     const ulonglong2 x = __ldg(p), y = __ldg(p + 1);
     if (x.x == key || x.y == key || y.x == key || y.y == key) return true;
-    if (x.x == kEmptyKey || x.y == kEmptyKey || y.x == kEmptyKey || y.y == kEmptyKey) return false;
+    // (keys fill a bucket left to right: the last slot is empty unless it is full)
+    if (y.y == kEmptyKey) return false;
     return has_edge_tail(h, key, bk);
 }
 
@@ -200,13 +203,16 @@ __device__ __forceinline__ bool group_any(bool f, const Groups& gr) {
 // Next-round task list: records [ns, cnt0, cnt1, graph, sid[ns], smc[ns],
 // frame[F_WORDS], list0[2 cnt0], list1[2 cnt1]] addressed by an index array.
 constexpr uint32_t kRecHeader = 4;
+constexpr uint32_t kTagShift = 40;   // Donation.tag
+constexpr uint32_t kDoneFlags = 32;  // Donation.done: flags, 128 bytes apart
 struct SplitBuf {
     uint32_t* words;
     unsigned long long* idx;
     int* refused;                 // first reason a split was refused (diagnostics; 0 = none)
     unsigned long long* used;     // words reserved (may pass word_cap: those failed)
     unsigned long long* count;    // records reserved (may pass idx_cap)
-    unsigned long long* count_fail;   // lowest record index whose reservation failed (~0: none)
+    unsigned long long* count_fail;   // complement of the lowest record index whose reservation
+                                      //   failed (0: none)
     unsigned long long word_cap;
     unsigned long long idx_cap;
 };
@@ -244,6 +250,9 @@ struct Ctx {
     unsigned long long work;                     // per-lane share
     uint32_t* sat;                               // shared: kSatCap per warp
     uint32_t* src;                               // shared: kSrcCap per warp
+    struct LaneShared* lanes;                    // shared: the last lane block's children
+    struct BitShared* bits;                      // shared: the bit search's part, or
+    struct LaneScratch* lane_scratch;            //   (the same words) the lane blocks'
     uint32_t lane;
 };
 
@@ -275,13 +284,13 @@ __device__ void flush(Ctx& t, const Outputs& o) {
 // A child or a node's scratch did not fit the arena.  Not an error yet: the
 // search loop moves the path into the next round's task list, where each
 // frame restarts at the bottom of an empty arena (run_dfs).
-// The failing frame and the site (1: a node's scratch, 2: a child) go to two
-// spare words after the warp's source list in shared memory, not to registers:
-// the search loop carries no extra state for this rare case.
+// The failing frame, the site (1: a node's scratch, 2: a child) and the child go
+// to spare words after the warp's source list in shared memory, not to
+// registers: the search loop carries no extra state for this rare case.
 constexpr int TASK_ARENA_FULL = 99;
 constexpr uint32_t kSiteNode = 1, kSiteChild = 2;
-__device__ __forceinline__ void arena_full(Ctx& t, uint32_t cur, uint32_t site) {
-    if (t.lane == 0) { t.src[kSrcCap] = cur; t.src[kSrcCap + 1] = site; }
+__device__ __forceinline__ void arena_full(Ctx& t, uint32_t cur, uint32_t site, uint32_t c) {
+    if (t.lane == 0) { t.src[kSrcCap] = cur; t.src[kSrcCap + 1] = site; t.src[kSrcCap + 2] = c; }
     __syncwarp();
     t.err = TASK_ARENA_FULL;
 }
@@ -700,7 +709,7 @@ __device__ bool emit(Ctx& t, const Outputs& o, const uint32_t* l0, uint32_t n0, 
             at = atomicAdd(o.out_pos, words);
             room = at + words <= o.out_cap;
             if (!room) {
-                atomicMin(o.out_fail, at);
+                atomicMax(o.out_fail, ~at);
             } else {
                 const unsigned long long c = atomicAdd(o.count, 1ull);
                 keep = !(o.limit && c >= o.limit);
@@ -747,12 +756,13 @@ __device__ bool emit(Ctx& t, const Outputs& o, const uint32_t* l0, uint32_t n0, 
     t.cnt++;
     t.hsum += final_h1(a, nx, ny);
     t.hxor ^= final_h2(b, nx, ny);
-    if (t.cnt >= kFlushBatch) flush(t, o);
     return true;
 }
 
 // ----------------------------------------------------------------- frames
 
+// A side that is global stores no list: its F_CNT / F_OFF words hold the
+// children left to be built one by one (bit i: id F_OFF + i; lane_blocks).
 struct Hdr {
     uint32_t ns, flags;
     U2 lo, cnt, off;
@@ -887,7 +897,7 @@ __device__ uint32_t build_child(Ctx& t, const Outputs& o, uint32_t cur, uint32_t
     const int os = 1 - s;
     const uint32_t nc = f.top;
     uint32_t w = nc + F_WORDS;
-    if (w > t.cap) { arena_full(t, cur, kSiteChild); return kNoPos; }
+    if (w > t.cap) { arena_full(t, cur, kSiteChild, c); return kNoPos; }
     Hdr ch;
     ch.ns = t.ns; ch.flags = 0; ch.lo.a = ch.lo.b = 0; ch.cnt.a = ch.cnt.b = 0; ch.off.a = ch.off.b = 0;
     ch.order = 0; ch.phase = 0; ch.pos = 0; ch.parent = cur; ch.end = 0xFFFFFFFFu;
@@ -905,7 +915,7 @@ __device__ uint32_t build_child(Ctx& t, const Outputs& o, uint32_t cur, uint32_t
             for (uint32_t i = 1; i < nsat; ++i)
                 if (degree(g, t.sat[i]) < degree(g, z)) z = t.sat[i];
             const uint32_t dz = degree(g, z);
-            if (w + 2ull * dz > t.cap) { arena_full(t, cur, kSiteChild); return kNoPos; }
+            if (w + 2ull * dz > t.cap) { arena_full(t, cur, kSiteChild, c); return kNoPos; }
             if (t.lane == 0) t.work += dz;
             const uint32_t* row = g.adj + g.off[z];
             #pragma unroll 1
@@ -934,7 +944,7 @@ __device__ uint32_t build_child(Ctx& t, const Outputs& o, uint32_t cur, uint32_t
     } else {
         const uint32_t* lst = t.arena + f.off.get(s);
         const uint32_t n = f.cnt.get(s);
-        if (w + 2ull * n > t.cap) { arena_full(t, cur, kSiteChild); return kNoPos; }
+        if (w + 2ull * n > t.cap) { arena_full(t, cur, kSiteChild, c); return kNoPos; }
         const uint32_t start = forced ? 0u : p + 1;
         // the frame's filter bitmaps, when it has them: sel = the rows of sat(c)
         const uint32_t* bm = nullptr;
@@ -1033,7 +1043,7 @@ __device__ uint32_t build_child(Ctx& t, const Outputs& o, uint32_t cur, uint32_t
             unsigned long long bound = 0;
             #pragma unroll 1
             for (uint32_t q = 0; q < nsrc; ++q) bound += degree(g, t.src[q]);
-            if (w + 2 * bound > t.cap) { arena_full(t, cur, kSiteChild); return kNoPos; }
+            if (w + 2 * bound > t.cap) { arena_full(t, cur, kSiteChild, c); return kNoPos; }
             #pragma unroll 1
             for (uint32_t q = 0; q < nsrc; ++q) {
                 const uint32_t m = t.src[q];
@@ -1064,7 +1074,7 @@ __device__ uint32_t build_child(Ctx& t, const Outputs& o, uint32_t cur, uint32_t
     } else {
         const uint32_t* lst = t.arena + f.off.get(os);
         const uint32_t n = f.cnt.get(os);
-        if (w + 2ull * n > t.cap) { arena_full(t, cur, kSiteChild); return kNoPos; }
+        if (w + 2ull * n > t.cap) { arena_full(t, cur, kSiteChild, c); return kNoPos; }
         #pragma unroll 1
         for (uint32_t base = 0; base < n; base += 32) {
             const uint32_t q = base + t.lane;
@@ -1094,344 +1104,77 @@ __device__ uint32_t build_child(Ctx& t, const Outputs& o, uint32_t cur, uint32_t
     return nc;
 }
 
-// ----------------------------------------------------------------- small subtrees
+// ----------------------------------------------------------------- task records
 
-// The subtree of a node whose sides are both local yields exactly the maximal
-// k-biplexes L with S ⊆ L ⊆ S ∪ C that have a V member: the node rules and
-// the branching only drop subsets of C that are no such L.  When C has at most
-// kSmallMax entries and S at most 32 members, solve_small tests every subset T
-// of C at once, one subset per lane, on bit masks, instead of walking the
-// subtree node by node:
-//  * S ∪ T is a k-biplex when every member misses at most k of the other side
-//    of S ∪ T: its misses inside S (smc, or the list's miss count for a
-//    candidate) plus popc(T & its candidate-miss mask);
-//  * it is maximal when no vertex outside it can join.  A vertex joins when it
-//    misses at most k of L's other side and none of those has k misses in L
-//    already (a blocker).  Left-out candidates are tested on their masks.  An
-//    outsider of side s that joins some L misses at most k members of S_o and
-//    no member with k misses inside S, so it lies in the row of such a
-//    saturated member (the lowest-degree one), or in one of the rows of any
-//    k + 1 members of S_o.  Those rows are scanned once; each outsider found
-//    is kept as two masks: the members of S_o and the candidates of C_o it
-//    misses.
-// Count mode hashes the results into the warp's counters.  Record mode
-// reserves room for all of the node's records at once (as emit does for one):
-// no room leaves everything untouched and the node is deferred to the next
-// round; then the results are counted (exact limit: past it, skip records)
-// and written.  Returns kSmallNo, having changed nothing, when the node does
-// not qualify: a side whose outsiders are not bounded that way (S_o has at
-// most k members, none saturated), source rows longer than kSmallScanMax in
-// total, too little arena room at `scratch` for the outsiders' masks, or (in
-// record mode) records that would fill more than half the record buffer.
-#ifndef GMK_SMALL_MAX
-#define GMK_SMALL_MAX 6
-#endif
-constexpr uint32_t kSmallMax = GMK_SMALL_MAX;   // 2^6 = 64 subsets: two per lane
-#ifndef GMK_SMALL_SCAN_MAX
-#define GMK_SMALL_SCAN_MAX 1024
-#endif
-constexpr uint32_t kSmallScanMax = GMK_SMALL_SCAN_MAX;   // outsider source-row entries
-constexpr int kSmallNo = 0, kSmallDone = 1, kSmallDefer = 2;
-
-__device__ __forceinline__ unsigned long long warp_xor64(unsigned long long v) {
-    #pragma unroll
-    for (int d = 16; d; d >>= 1) v ^= __shfl_xor_sync(kFull, v, d);
-    return v;
-}
-
-// Inclusive warp prefix sum.
-__device__ __forceinline__ uint32_t warp_scan(uint32_t v, uint32_t lane) {
-    #pragma unroll
-    for (uint32_t d = 1; d < 32; d <<= 1) {
-        const uint32_t x = __shfl_up_sync(kFull, v, d);
-        if (lane >= d) v += x;
-    }
-    return v;
-}
-
-template <bool kRec>
-__device__ __forceinline__ int solve_small(Ctx& t, const Outputs& o, const uint32_t* l0, uint32_t n0,
-                                           const uint32_t* l1, uint32_t n1, uint32_t scratch) {
-    const GraphView& g = t.g;
-    const uint32_t ns = t.ns, m = n0 + n1, k = t.k, lane = t.lane;
-    // lane i < ns holds member i, lane j < m candidate j (list 0, then list 1)
-    const bool is_mem = lane < ns;
-    const uint32_t my_v = is_mem ? t.sid[lane] : 0u;
-    const uint32_t my_smc = is_mem ? t.smc[lane] : 0u;
-    const uint32_t mem1 = __ballot_sync(kFull, is_mem && side_of(g, my_v));
-    const uint32_t mem0 = __ballot_sync(kFull, is_mem) & ~mem1;
-    const bool is_cand = lane < m;
-    const bool c_one = lane >= n0;
-    const uint32_t* lc = c_one ? l1 + 2 * (lane - n0) : l0 + 2 * lane;
-    const uint32_t my_c = is_cand ? lc[0] : 0u;
-    const uint32_t my_cm = is_cand ? lc[1] : 0u;
-    const uint32_t cand0 = (1u << n0) - 1u;
-    const uint32_t cand1 = ((1u << m) - 1u) & ~cand0;
-
-    // outsider sources per outsider side s, as member masks of S_o
-    unsigned long long key0 = ~0ull, key1 = ~0ull;
-    if (is_mem && my_smc >= k) {
-        const unsigned long long key = ((unsigned long long)degree(g, my_v) << 32) | lane;
-        if (side_of(g, my_v)) key1 = key; else key0 = key;
-    }
-    key0 = warp_min64(key0);
-    key1 = warp_min64(key1);
-    uint32_t srcm[2];
-    uint32_t total = 0;
-    #pragma unroll 1
-    for (int s = 0; s < 2; ++s) {
-        const unsigned long long key = s ? key0 : key1;   // side o = 1 - s
-        uint32_t memo = s ? mem0 : mem1;
-        uint32_t sm = 0;
-        if (key != ~0ull) {
-            sm = 1u << (uint32_t)key;
+// Reserves `words` words and `recs` index slots of the next round's task list
+// (warp-uniform result).  Reservations are plain atomic adds: thousands of
+// warps split at once when a round winds down.  Positions only grow, so once
+// one reservation fails every later one fails too: the records below
+// that one are the complete, written ones.  A failed word reservation is
+// simply left unused.
+__device__ bool reserve_records(Ctx& t, const SplitBuf& sb, unsigned long long words,
+                                unsigned long long recs, unsigned long long* w0_out,
+                                unsigned long long* r0_out) {
+    unsigned long long w0 = 0, r0 = 0;
+    int ok = 0;
+    if (t.lane == 0) {
+        w0 = atomicAdd(sb.used, words);
+        if (w0 + words <= sb.word_cap) {
+            r0 = atomicAdd(sb.count, recs);
+            if (r0 + recs <= sb.idx_cap) ok = 1;
+            else { atomicMax(sb.count_fail, ~r0); atomicCAS(sb.refused, 0, 4); }
         } else {
-            if ((uint32_t)__popc(memo) < k + 1) return kSmallNo;
-            #pragma unroll 1
-            for (uint32_t c = 0; c <= k; ++c) { sm |= memo & (0u - memo); memo &= memo - 1; }
-        }
-        srcm[s] = sm;
-        #pragma unroll 1
-        for (uint32_t x = sm; x; x &= x - 1) total += degree(g, __shfl_sync(kFull, my_v, __ffs(x) - 1));
-    }
-    if (total > kSmallScanMax || scratch + 2ull * total > t.cap) return kSmallNo;
-
-    // candidate j: the other side's candidates and members it misses
-    uint32_t my_mcc = 0, my_mcs = 0;
-    #pragma unroll 1
-    for (uint32_t j = 0; j < m; ++j) {
-        const uint32_t cj = __shfl_sync(kFull, my_c, j);
-        if (is_cand && c_one != (j >= n0) && !has_edge(t.eh, my_c, cj)) my_mcc |= 1u << j;
-    }
-    #pragma unroll 1
-    for (uint32_t x = c_one ? mem0 : mem1, y = mem0 | mem1; y; y &= y - 1) {
-        const uint32_t i = __ffs(y) - 1;
-        const uint32_t vi = __shfl_sync(kFull, my_v, i);
-        if (is_cand && ((x >> i) & 1u) && !has_edge(t.eh, my_c, vi)) my_mcs |= 1u << i;
-    }
-    // member i: the candidates it misses (the transpose of the above)
-    uint32_t my_msc = 0;
-    #pragma unroll 1
-    for (uint32_t j = 0; j < m; ++j)
-        if ((__shfl_sync(kFull, my_mcs, j) >> lane) & 1u) my_msc |= 1u << j;
-
-    // outsiders: masks (members of S_o missed, candidates of C_o missed)
-    uint32_t* ob = t.arena + scratch;
-    uint32_t n_out = 0;
-    #pragma unroll 1
-    for (int s = 0; s < 2; ++s) {
-        const uint32_t mems = s ? mem1 : mem0, memo = s ? mem0 : mem1;
-        const uint32_t cands = s ? cand1 : cand0, cando = s ? cand0 : cand1;
-        uint32_t seen_src = 0;
-        #pragma unroll 1
-        for (uint32_t sm = srcm[s]; sm; sm &= sm - 1) {
-            const uint32_t qi = __ffs(sm) - 1;
-            const uint32_t src = __shfl_sync(kFull, my_v, qi);
-            const uint32_t d = degree(g, src);
-            const uint32_t* row = g.adj + g.off[src];
-            #pragma unroll 1
-            for (uint32_t base = 0; base < d; base += 32) {
-                const uint32_t p = base + lane;
-                bool keep = p < d;
-                const uint32_t e = keep ? row[p] : 0u;
-                // in S_s or C_s: not an outsider (every shuffle is taken by
-                // all lanes: none sits behind a short-circuit)
-                #pragma unroll 1
-                for (uint32_t y = mems; y; y &= y - 1) {
-                    const uint32_t vi = __shfl_sync(kFull, my_v, __ffs(y) - 1);
-                    keep = keep && vi != e;
-                }
-                #pragma unroll 1
-                for (uint32_t y = cands; y; y &= y - 1) {
-                    const uint32_t cj = __shfl_sync(kFull, my_c, __ffs(y) - 1);
-                    keep = keep && cj != e;
-                }
-                // found at an earlier source already
-                #pragma unroll 1
-                for (uint32_t y = seen_src; y; y &= y - 1) {
-                    const uint32_t vr = __shfl_sync(kFull, my_v, __ffs(y) - 1);
-                    keep = keep && !has_edge(t.eh, e, vr);
-                }
-                // misses against S_o: at most k, none on a member with k misses
-                uint32_t mos = 0;
-                #pragma unroll 1
-                for (uint32_t y = memo; y; y &= y - 1) {
-                    const uint32_t i = __ffs(y) - 1;
-                    const uint32_t vi = __shfl_sync(kFull, my_v, i);
-                    const uint32_t si = __shfl_sync(kFull, my_smc, i);
-                    if (keep && !has_edge(t.eh, e, vi)) {
-                        mos |= 1u << i;
-                        keep = si < k && (uint32_t)__popc(mos) <= k;
-                    }
-                }
-                uint32_t moc = 0;
-                #pragma unroll 1
-                for (uint32_t y = cando; y; y &= y - 1) {
-                    const uint32_t j = __ffs(y) - 1;
-                    const uint32_t cj = __shfl_sync(kFull, my_c, j);
-                    if (keep && !has_edge(t.eh, e, cj)) moc |= 1u << j;
-                }
-                const uint32_t km = __ballot_sync(kFull, keep);
-                if (keep) {
-                    const uint32_t r = n_out + __popc(km & lanemask_lt());
-                    ob[2 * r] = mos;
-                    ob[2 * r + 1] = moc;
-                }
-                n_out += __popc(km);
-            }
-            seen_src |= 1u << qi;
+            atomicCAS(sb.refused, 0, 3);
         }
     }
-    __syncwarp();
-
-    // hash elements: S's sums, and each candidate's
-    unsigned long long ea = is_mem ? elem_a(my_v) : 0ull;
-    const unsigned long long a_s = warp_sum64(ea);
-    const unsigned long long b_s = warp_sum64(is_mem ? elem_b(ea) : 0ull);
-    const unsigned long long my_ea = is_cand ? elem_a(my_c) : 0ull;
-    const unsigned long long my_eb = is_cand ? elem_b(my_ea) : 0ull;
-
-    // every subset T of C, one per lane; found bit r: subset 32 r + lane is a result
-    unsigned long long cnt = 0, h1 = 0, h2 = 0;
-    uint32_t found = 0;
-    const uint32_t nsub = 1u << m;
-    #pragma unroll 1
-    for (uint32_t base = 0; base < nsub; base += 32) {
-        const uint32_t T = base + lane;
-        bool alive = T < nsub && t.nss.b + __popc(T & cand1) > 0;   // a V member
-        uint32_t bs = 0, bt = 0;
-        #pragma unroll 1
-        for (uint32_t y = mem0 | mem1; y; y &= y - 1) {
-            const uint32_t i = __ffs(y) - 1;
-            const uint32_t tt = __shfl_sync(kFull, my_smc, i) + __popc(T & __shfl_sync(kFull, my_msc, i));
-            alive = alive && tt <= k;
-            bs |= tt >= k ? 1u << i : 0u;
-        }
-        #pragma unroll 1
-        for (uint32_t j = 0; j < m; ++j) {
-            const uint32_t tt = __shfl_sync(kFull, my_cm, j) + __popc(T & __shfl_sync(kFull, my_mcc, j));
-            if ((T >> j) & 1u) {
-                alive = alive && tt <= k;
-                bt |= tt >= k ? 1u << j : 0u;
-            }
-        }
-        // left-out candidates, then outsiders: none may join
-        #pragma unroll 1
-        for (uint32_t j = 0; j < m; ++j) {
-            const uint32_t mcc = __shfl_sync(kFull, my_mcc, j);
-            const uint32_t mcs = __shfl_sync(kFull, my_mcs, j);
-            const uint32_t cm = __shfl_sync(kFull, my_cm, j);
-            if (!((T >> j) & 1u) && cm + __popc(T & mcc) <= k && !(mcs & bs) && !(mcc & bt))
-                alive = false;
-        }
-        #pragma unroll 1
-        for (uint32_t x = 0; x < n_out; ++x) {
-            if ((x & 15u) == 0 && !__any_sync(kFull, alive)) break;
-            const uint32_t mos = ob[2 * x], moc = ob[2 * x + 1];
-            if (__popc(mos) + __popc(T & moc) <= k && !(mos & bs) && !(moc & bt)) alive = false;
-        }
-        if (alive) found |= 1u << (base >> 5);
-        if (kRec || !__any_sync(kFull, alive)) continue;
-        unsigned long long a = a_s, b = b_s;
-        #pragma unroll 1
-        for (uint32_t j = 0; j < m; ++j) {
-            const unsigned long long aj = __shfl_sync(kFull, my_ea, j);
-            const unsigned long long bj = __shfl_sync(kFull, my_eb, j);
-            if ((T >> j) & 1u) { a += aj; b += bj; }
-        }
-        if (alive) {
-            const uint32_t nx = t.nss.a + __popc(T & cand0), ny = t.nss.b + __popc(T & cand1);
-            cnt += 1;
-            h1 += final_h1(a, nx, ny);
-            h2 ^= final_h2(b, nx, ny);
-        }
-    }
-    if (!kRec) {
-        t.cnt += warp_sum64(cnt);
-        t.hsum += warp_sum64(h1);
-        t.hxor ^= warp_xor64(h2);
-        return kSmallDone;
-    }
-    // record mode: room for every record of the node first, then the count
-    uint32_t nres = __popc(found), words = 0;
-    #pragma unroll 1
-    for (uint32_t x = found; x; x &= x - 1) {
-        const uint32_t T = ((__ffs(x) - 1) << 5) + lane;
-        words += 2 + ns + __popc(T);
-    }
-    uint32_t rank = warp_scan(nres, lane), off = warp_scan(words, lane);
-    const uint32_t n_res = __shfl_sync(kFull, rank, 31), n_words = __shfl_sync(kFull, off, 31);
-    rank -= nres;
-    off -= words;
-    if (n_res == 0) return kSmallDone;
-    // records that would fill more than half the buffer go one by one (emit)
-    // down the usual path: a node must never need more room than a drained
-    // buffer has
-    if (2ull * n_words > o.out_cap) return kSmallNo;
-    unsigned long long at = 0, c0 = 0;
-    int room = 0;
-    if (lane == 0) {
-        at = atomicAdd(o.out_pos, (unsigned long long)n_words);
-        room = at + n_words <= o.out_cap;
-        if (!room) {
-            atomicMin(o.out_fail, at);
-        } else {
-            c0 = atomicAdd(o.count, (unsigned long long)n_res);
-            if (o.limit && c0 + n_res >= o.limit) atomicExch(o.stop, 1);
-        }
-    }
-    if (!bcast(room)) return kSmallDefer;
-    at = bcast(at);
-    c0 = bcast(c0);
-    #pragma unroll 1
-    for (uint32_t base = 0; base < nsub; base += 32) {
-        const uint32_t T = base + lane;
-        unsigned long long a = a_s, b = b_s;
-        #pragma unroll 1
-        for (uint32_t j = 0; j < m; ++j) {
-            const unsigned long long aj = __shfl_sync(kFull, my_ea, j);
-            const unsigned long long bj = __shfl_sync(kFull, my_eb, j);
-            if ((T >> j) & 1u) { a += aj; b += bj; }
-        }
-        if (!((found >> (base >> 5)) & 1u)) continue;
-        const uint32_t nx = t.nss.a + __popc(T & cand0), ny = t.nss.b + __popc(T & cand1);
-        uint32_t* r = o.out_buf + at + off;
-        off += 2 + nx + ny;
-        if (o.limit && c0 + rank++ >= o.limit) {
-            // past the limit: a skip record of the same length
-            r[0] = 0xFFFFFFFFu;
-            r[1] = nx + ny;
-            continue;
-        }
-        h1 += final_h1(a, nx, ny);
-        h2 ^= final_h2(b, nx, ny);
-        r[0] = nx;
-        r[1] = ny;
-        uint32_t px = 2, py = 2 + nx;
-        #pragma unroll 1
-        for (uint32_t i = 0; i < ns; ++i) {
-            const uint32_t v = t.sid[i];
-            if (side_of(g, v)) r[py++] = v; else r[px++] = v;
-        }
-        #pragma unroll 1
-        for (uint32_t j = 0; j < m; ++j)
-            if ((T >> j) & 1u) {
-                if (j < n0) r[px++] = l0[2 * j];
-                else r[py++] = l1[2 * (j - n0)];
-            }
-    }
-    h1 = warp_sum64(h1);
-    h2 = warp_xor64(h2);
-    if (lane == 0) {
-        atomicAdd(o.hash_sum, h1);
-        atomicXor(o.hash_xor, h2);
-    }
-    __syncwarp();
-    return kSmallDone;
+    if (!bcast(ok)) return false;
+    *w0_out = bcast(w0);
+    *r0_out = bcast(r0);
+    return true;
 }
+
+// In-launch work sharing.  A warp that runs out of tasks takes a ticket t (a
+// counter) and waits on slot t of the record index.  A busy warp that sees
+// more tickets than reserved slots (at its poll points) splits the shallowest
+// frame of its path that still has unexplored children: the first half of
+// that frame's remaining children in the current phase goes into a record
+// (F_POS .. F_END, one phase only), the warp keeps the rest.  So the work
+// spreads by halving, and each waiting warp watches its own slot -- no retry
+// loops on shared counters.  `outstanding` counts the launch's unfinished
+// tasks (the queue's entries plus the donations, minus the finished), offset
+// by the queue length: the launch's work is done when it is -queue_len, and the
+// warp that makes it so tells the waiting ones through `done` flags (one line
+// for every 32nd warp: thousands of warps polling one counter would slow its
+// atomics, and polling it rarely would keep them past the end).
+// Records live in a bump-allocated buffer for the launch; once it is full,
+// donation stops and busy warps split into the next round as before.
+struct Donation {
+    uint32_t* words;
+    unsigned long long word_cap;
+    unsigned long long* idx;          // slot -> tag | record offset + 1; another tag: not yet written
+    unsigned long long tag;           // this launch's number, in bits 40 and up
+    unsigned long long idx_cap;
+    unsigned long long* used;         // words reserved
+    unsigned long long* tail;         // slots reserved
+    unsigned long long* claim;        // tickets taken by waiting warps
+    unsigned long long* outstanding;  // unfinished tasks - queue_len (mod 2^64)
+    unsigned long long* donated;      // records published (statistics)
+    int* full;                        // a reservation failed: no more donations
+    int* done;                        // kDoneFlags flags: the launch's work is done
+    uint32_t min_nodes;               // a task donates only after this many nodes
+};
+
+}  // namespace warp
+}  // namespace gmk
+#include "enum_bits.cuh"
+#include "enum_lanes.cuh"
+namespace gmk {
+namespace warp {
 
 // enter_node: the node's result record found no room in the record buffer.
 constexpr int ENTER_DEFER = 3;
+// enter_node: the node goes to the bit-mask search; its universe is collected.
+constexpr int ENTER_BITS = 4;
 
 // The child a node asks for: "S + c", c on side s at list position p.
 struct ChildReq {
@@ -1443,7 +1186,8 @@ struct ChildReq {
 // Warp form of enter_node (enum_core.cuh).  ENTER_PUSHED: a forced candidate
 // was found; *req describes the child to build.
 template <bool kRec, bool kBits>
-__device__ int enter_node(Ctx& t, const Outputs& o, uint32_t cur, ChildReq* req) {
+__device__ int enter_node(Ctx& t, const Outputs& o, uint32_t cur, ChildReq* req, Bits& bits,
+                          BitSources& src) {
     const GraphView& g = t.g;
     const Hdr f = read_hdr(t.arena + cur);
     pop_to(t, f.ns);
@@ -1453,7 +1197,7 @@ __device__ int enter_node(Ctx& t, const Outputs& o, uint32_t cur, ChildReq* req)
         const int s = g0 ? 0 : 1, os = 1 - s;
         const uint32_t n = f.cnt.get(os);
         const uint32_t base = f.top;
-        if (base + n + 2ull * t.ns > t.cap) { arena_full(t, cur, kSiteNode); return ENTER_DONE; }
+        if (base + n + 2ull * t.ns > t.cap) { arena_full(t, cur, kSiteNode, 0); return ENTER_DONE; }
         if (outsider_addable_mixed(t, s, f.lo.get(s), t.arena + f.off.get(os), n, t.arena + base))
             return ENTER_DONE;
     }
@@ -1464,8 +1208,11 @@ __device__ int enter_node(Ctx& t, const Outputs& o, uint32_t cur, ChildReq* req)
         const unsigned long long pairs = (unsigned long long)(t.ns + n0) * (t.ns + n1);
         if (n0 + n1 == 0 || pairs <= t.scan_limit) {
             const uint32_t base = f.top;
+            if (t.nss.a + n0 <= kBitsSide && t.nss.b + n1 <= kBitsSide &&
+                bits_collect(t, bits, src, l0, n0, l1, n1, base))
+                return ENTER_BITS;
             if (base + (unsigned long long)t.ns + n0 + n1 > t.cap) {
-                arena_full(t, cur, kSiteNode);
+                arena_full(t, cur, kSiteNode, 0);
                 return ENTER_DONE;
             }
             uint32_t* tot = t.arena + base;
@@ -1532,16 +1279,6 @@ __device__ int enter_node(Ctx& t, const Outputs& o, uint32_t cur, ChildReq* req)
                 return ENTER_DONE;
             }
             if (addable) return ENTER_DONE;
-            // a small candidate set: every subset at once (solve_small; in the
-            // k = 1 kernels only -- the k >= 2 ones ran 5-25 % slower with it)
-            if (!kBits && n0 + n1 <= kSmallMax && t.ns <= 32) {
-                const int r = solve_small<kRec>(t, o, l0, n0, l1, n1, base + t.ns + n0 + n1);
-                if (r == kSmallDefer) return ENTER_DEFER;
-                if (r == kSmallDone) {
-                    if (!kRec && t.cnt >= kFlushBatch) flush(t, o);
-                    return ENTER_DONE;
-                }
-            }
             // forced candidate: fits every leaf that lacks it (first in list order)
             #pragma unroll 1
             for (int s = 0; s < 2; ++s) {
@@ -1604,35 +1341,52 @@ __device__ int enter_node(Ctx& t, const Outputs& o, uint32_t cur, ChildReq* req)
     return ENTER_ITERATE;
 }
 
+enum : int { NEXT_NONE = 0, NEXT_CHILD = 1, NEXT_BLOCK = 2 };
+
 // Warp form of next_child (enum_core.cuh): advances frame cur to its next
-// child and describes it in *req; false when the frame is finished.
-__device__ bool next_child(Ctx& t, uint32_t cur, ChildReq* req) {
+// child and describes it in *req.  The children of a global side are first
+// looked at in blocks (lane_blocks): NEXT_BLOCK says that one is due (*hdr the
+// frame's header, req->s the side, req->opp_done), and the children that it
+// leaves to be built come one by one.  NEXT_NONE: the frame is finished.
+// `blocks` false (the plain schedule): every child comes one by one.
+__device__ int next_child(Ctx& t, uint32_t cur, bool blocks, ChildReq* req, Hdr* hdr) {
     const GraphView& g = t.g;
     uint32_t* f = t.arena + cur;
     const Hdr h = read_hdr(f);
     uint32_t phase = h.phase, pos = h.pos;
+    req->forced = false;
     while (phase < 2) {
         const int s = phase == 0 ? (int)h.order : 1 - (int)h.order;
         const bool opp_done = phase == 1;
-        uint32_t c = 0, p = kNoPos;
-        bool have = false;
+        uint32_t c = 0, p = kNoPos, pend;
+        int have = NEXT_NONE;
         // F_END bounds the current phase's positions: a root chunk's last
         // V child, or the end of a donated range of children
         if (h.flags & gbit(s)) {
             const uint32_t end = h.end < side_end(g, s) ? h.end : side_end(g, s);
-            if (pos < end) { c = pos; p = kNoPos; ++pos; have = true; }
+            pend = h.cnt.get(s);
+            if (pend && !(h.flags & FL_BUILD)) {
+                have = NEXT_BLOCK;       // to be looked at again: handed on by another warp
+            } else if (pend) {
+                c = h.off.get(s) + (uint32_t)__ffs(pend) - 1;
+                if (t.lane == 0) f[F_CNT0 + s] = pend & (pend - 1);
+                have = NEXT_CHILD;
+            } else if (pos < end) {
+                if (!blocks) { c = pos; ++pos; }
+                have = blocks ? NEXT_BLOCK : NEXT_CHILD;
+            }
         } else if (pos < (h.end < h.cnt.get(s) ? h.end : h.cnt.get(s))) {
             p = pos;
             c = t.arena[h.off.get(s) + 2 * p];
             ++pos;
-            have = true;
+            have = NEXT_CHILD;
         }
         // U children after the V side is exhausted need a V member in S
         if (have && opp_done && s == 0) {
             bool anyv = false;
             #pragma unroll 1
             for (uint32_t i = t.lane; i < h.ns; i += 32) anyv |= side_of(g, t.sid[i]) != 0;
-            if (!__any_sync(kFull, anyv)) { have = false; phase = 2; }
+            if (!__any_sync(kFull, anyv)) { have = NEXT_NONE; phase = 2; }
         }
         if (!have) {
             if (phase == 2) break;
@@ -1644,18 +1398,21 @@ __device__ bool next_child(Ctx& t, uint32_t cur, ChildReq* req) {
             }
             continue;
         }
-        if (t.lane == 0) { f[F_PHASE] = phase; f[F_POS] = pos; }
-        __syncwarp();
         req->c = c;
         req->s = s;
         req->p = p;
-        req->forced = false;
         req->opp_done = opp_done;
-        return true;
+        if (have == NEXT_BLOCK) {
+            *hdr = h;
+            hdr->pos = pos;
+        }
+        if (t.lane == 0) { f[F_PHASE] = phase; f[F_POS] = pos; }
+        __syncwarp();
+        return have;
     }
     if (t.lane == 0) { f[F_PHASE] = phase; f[F_POS] = pos; }
     __syncwarp();
-    return false;
+    return NEXT_NONE;
 }
 
 // ----------------------------------------------------------------- splitting
@@ -1671,33 +1428,6 @@ __device__ __forceinline__ uint32_t frame_list_words(const uint32_t* f) {
     const uint32_t c0 = (f[F_FLAGS] & FL_G0) ? 0u : f[F_CNT0];
     const uint32_t c1 = (f[F_FLAGS] & FL_G1) ? 0u : f[F_CNT1];
     return 2 * (c0 + c1);
-}
-
-// Reserves `words` words and `recs` index slots of the next round's task list
-// (warp-uniform result).  Reservations are plain atomic adds: thousands of
-// warps split at once when a round winds down.  Positions only grow, so once
-// one reservation fails every later one fails too: the records below
-// count_fail are the complete, written ones.  A failed word reservation is
-// simply left unused.
-__device__ bool reserve_records(Ctx& t, const SplitBuf& sb, unsigned long long words,
-                                unsigned long long recs, unsigned long long* w0_out,
-                                unsigned long long* r0_out) {
-    unsigned long long w0 = 0, r0 = 0;
-    int ok = 0;
-    if (t.lane == 0) {
-        w0 = atomicAdd(sb.used, words);
-        if (w0 + words <= sb.word_cap) {
-            r0 = atomicAdd(sb.count, recs);
-            if (r0 + recs <= sb.idx_cap) ok = 1;
-            else { atomicMin(sb.count_fail, r0); atomicCAS(sb.refused, 0, 4); }
-        } else {
-            atomicCAS(sb.refused, 0, 3);
-        }
-    }
-    if (!bcast(ok)) return false;
-    *w0_out = bcast(w0);
-    *r0_out = bcast(r0);
-    return true;
 }
 
 // Copies a record of this round unchanged into the next round's task list
@@ -1771,50 +1501,34 @@ __device__ bool split_path(Ctx& t, const SplitBuf& sb, uint32_t cur) {
 
 // ----------------------------------------------------------------- work sharing
 
-// In-launch work sharing.  A warp that runs out of tasks takes a ticket t (a
-// counter) and waits on slot t of the record index.  A busy warp that sees
-// more tickets than reserved slots (at its poll points) splits the shallowest
-// frame of its path that still has unexplored children: the first half of
-// that frame's remaining children in the current phase goes into a record
-// (F_POS .. F_END, one phase only), the warp keeps the rest.  So the work
-// spreads by halving, and each waiting warp watches its own slot -- no retry
-// loops on shared counters.  `outstanding` counts the launch's unfinished
-// tasks (the queue's entries plus the donations, minus the finished), offset
-// by the queue length: the launch's work is done when it is -queue_len.
-// Records live in a bump-allocated buffer for the launch; once it is full,
-// donation stops and busy warps split into the next round as before.
-struct Donation {
-    uint32_t* words;
-    unsigned long long word_cap;
-    unsigned long long* idx;          // slot -> record offset + 1 (0: not yet written)
-    unsigned long long idx_cap;
-    unsigned long long* used;         // words reserved
-    unsigned long long* tail;         // slots reserved
-    unsigned long long* claim;        // tickets taken by waiting warps
-    unsigned long long* outstanding;  // unfinished tasks - queue_len (mod 2^64)
-    unsigned long long* donated;      // records published (statistics)
-    int* full;                        // a reservation failed: no more donations
-    uint32_t min_nodes;               // a task donates only after this many nodes
-};
-
-// Positions left in the current phase of entered frame f ([pos, lim)), and
-// whether a second phase follows.
+// Positions left in the current phase of entered frame f ([pos, lim)), its
+// pending children, and whether a second phase follows.
 struct Rest {
-    uint32_t pos, lim;
+    uint32_t pos, lim, pend;
+    bool by_block;      // a global side: its range is handed out in blocks of 32
     bool next_phase;
+    // anything to hand out?  (a range of one block stays; the second phase goes
+    // only when the first is used up)
+    __device__ __forceinline__ bool range() const { return lim - pos > (by_block ? 32u : 0u); }
+    __device__ __forceinline__ bool any() const {
+        return range() || pend || (lim == pos && next_phase);
+    }
 };
 
 __device__ __forceinline__ Rest frame_rest(const GraphView& g, const uint32_t* f) {
-    Rest r{0, 0, false};
+    Rest r{0, 0, 0, false, false};
     const uint32_t phase = f[F_PHASE];
     if (phase >= 2) return r;
     const uint32_t order = f[F_ORDER];
     const int s = phase == 0 ? (int)order : 1 - (int)order;
     const uint32_t flags = f[F_FLAGS];
-    const uint32_t side = (flags & (s ? FL_G1 : FL_G0)) ? side_end(g, s) : f[F_CNT0 + s];
+    const bool global = flags & (s ? FL_G1 : FL_G0);
+    const uint32_t side = global ? side_end(g, s) : f[F_CNT0 + s];
     r.pos = f[F_POS];
     r.lim = f[F_END] < side ? f[F_END] : side;
     if (r.pos > r.lim) r.pos = r.lim;
+    r.by_block = global;
+    r.pend = global ? f[F_CNT0 + s] : 0u;
     if (phase == 0 && !(flags & FL_ONE_PHASE)) {
         const int s2 = 1 - s;
         r.next_phase = (flags & (s2 ? FL_G1 : FL_G0)) ? f[F_LO0 + s2] + 1 < side_end(g, s2)
@@ -1838,13 +1552,13 @@ constexpr uint32_t kMaxDonateParts = GMK_DONATE_PARTS;
 __device__ __forceinline__ bool donate_top(Ctx& t, const Donation& db, uint32_t cur,
                                            unsigned long long want) {
     uint32_t best = kNoPos;
-    Rest rb{0, 0, false};
+    Rest rb{0, 0, 0, false, false};
     #pragma unroll 1
     for (uint32_t x = cur; x != kNoPos; x = t.arena[x + F_PARENT_SLOT]) {
         const uint32_t* f = t.arena + x;
         if (!(f[F_FLAGS] & FL_ENTERED)) continue;
         const Rest r = frame_rest(t.g, f);
-        if (r.lim > r.pos || r.next_phase) { best = x; rb = r; }
+        if (r.any()) { best = x; rb = r; }
     }
     if (best == kNoPos) return false;
     const uint32_t* f = t.arena + best;
@@ -1856,7 +1570,11 @@ __device__ __forceinline__ bool donate_top(Ctx& t, const Donation& db, uint32_t 
     // current phase's remaining children (one record takes half; with many
     // warps waiting, up to kMaxDonateParts records of equal shares), the
     // donor keeps the rest
-    const uint32_t rem = rb.lim - rb.pos;
+    // (a global side's range is split in blocks of 32 children, which cost
+    // lane_blocks as much as one; the children it left pending by their mask)
+    const bool by_range = rb.range(), by_mask = !by_range && rb.pend != 0;
+    const uint32_t unit = rb.by_block ? 32u : 1u;
+    const uint32_t rem = by_range ? (rb.lim - rb.pos + unit - 1) / unit : by_mask ? __popc(rb.pend) : 0u;
     uint32_t parts = 1;
     if (rem >= 3 && want > 1) {
         const unsigned long long cap = want < kMaxDonateParts ? want : kMaxDonateParts;
@@ -1876,11 +1594,16 @@ __device__ __forceinline__ bool donate_top(Ctx& t, const Donation& db, uint32_t 
     w0 = bcast(w0);
     slot = bcast(slot);
     uint32_t r_phase = f[F_PHASE], r_pos = rb.pos, q = 1, r_flags = f[F_FLAGS], r_end = 0;
-    uint32_t keep_phase = f[F_PHASE], keep_pos;
+    uint32_t keep_phase = f[F_PHASE], keep_pos, keep_pend = rb.pend;
+    // the side that the current phase iterates; a record of a global one
+    // carries its own part of the pending children
+    const uint32_t r_side = keep_phase == 0 ? f[F_ORDER] : 1u - f[F_ORDER];
+    const bool r_global = f[F_FLAGS] & (r_side ? FL_G1 : FL_G0);
     if (rem >= 1) {
         q = rem >= 2 ? rem / (parts + 1) : 1u;
+        if (by_range) q *= unit;
         r_flags |= FL_ONE_PHASE;
-        keep_pos = rb.pos + parts * q;
+        keep_pos = by_mask ? f[F_POS] : rb.pos + parts * q;
     } else {
         // the current phase is used up: the record takes the second phase
         const int s2 = f[F_ORDER] ? 0 : 1;
@@ -1924,11 +1647,19 @@ __device__ __forceinline__ bool donate_top(Ctx& t, const Donation& db, uint32_t 
     #pragma unroll 1
     for (uint32_t pp = 0; pp < parts; ++pp) {
         uint32_t* fr = r + pp * words + kRecHeader + 2 * ns;
+        uint32_t part_mask = 0;   // the next q pending children
+        if (by_mask) {
+            const uint32_t before = keep_pend;
+            #pragma unroll 1
+            for (uint32_t i = 0; i < q; ++i) keep_pend &= keep_pend - 1;
+            part_mask = before & ~keep_pend;
+        }
         if (t.lane < F_WORDS) {
             uint32_t v = f[t.lane];
             v = t.lane == F_PHASE ? r_phase : v;
-            v = t.lane == F_POS ? (rem >= 1 ? r_pos + pp * q : r_pos) : v;
-            v = t.lane == F_END ? (rem >= 1 ? r_pos + (pp + 1) * q : r_end) : v;
+            v = t.lane == F_POS ? (rem >= 1 && !by_mask ? r_pos + pp * q : r_pos) : v;
+            v = t.lane == F_END ? (by_mask ? r_pos : rem >= 1 ? r_pos + (pp + 1) * q : r_end) : v;
+            v = t.lane == F_CNT0 + r_side && r_global ? part_mask : v;
             v = t.lane == F_FLAGS ? r_flags : v;
             fr[t.lane] = v;
         }
@@ -1945,9 +1676,10 @@ __device__ __forceinline__ bool donate_top(Ctx& t, const Donation& db, uint32_t 
         atomicAdd(db.donated, (unsigned long long)parts);
         __threadfence();
         #pragma unroll 1
-        for (uint32_t pp = 0; pp < parts; ++pp) atomicExch(db.idx + slot + pp, w0 + pp * words + 1);
+        for (uint32_t pp = 0; pp < parts; ++pp) atomicExch(db.idx + slot + pp, db.tag | (w0 + pp * words + 1));
         t.arena[best + F_PHASE] = keep_phase;   // the donor keeps the rest
         t.arena[best + F_POS] = keep_pos;
+        if (by_mask) t.arena[best + F_CNT0 + r_side] = keep_pend;
     }
     __syncwarp();
     return true;
@@ -1957,6 +1689,7 @@ __device__ __forceinline__ bool donate_top(Ctx& t, const Donation& db, uint32_t 
 
 struct RunLimits {
     uint32_t split_min_nodes;           // 0: never split for load balance
+    bool blocks;                        // children of a global side go through lane_blocks
     const unsigned long long* queue;    // the round's queue head
     unsigned long long queue_len;       // entries this warp's round hands out
     // record mode: once *out_pos passes drain_at the round winds down -- every
@@ -1971,7 +1704,8 @@ __device__ __forceinline__ bool draining(const RunLimits& lim) {
 }
 
 // Depth-first search from the frame at arena offset 0; returns the nodes it
-// entered.
+// entered.  One loop step looks at one thing: a few states of the bit search,
+// one node, one block of children, or one child.
 template <bool kRec, bool kBits>
 __device__ __forceinline__ unsigned long long run_dfs(Ctx& t, const Outputs& o, uint32_t first,
                                                      const SplitBuf* sb, const RunLimits& lim,
@@ -1980,12 +1714,39 @@ __device__ __forceinline__ unsigned long long run_dfs(Ctx& t, const Outputs& o, 
     uint32_t polls = 0;
     unsigned long long task_nodes = 0;
     bool may_split = sb != nullptr && (lim.split_min_nodes != 0 || lim.drain_at != 0);
-    while (cur != kNoPos) {
+    // a path, or the bit search's states, to be moved to the next round, and
+    // the error if that fails (0: none, the work goes on here)
+    uint32_t split_at = kNoPos;
+    int split_fail = 0;
+    bool bits_out = false;
+    Bits bits;
+    bits.active = false;
+    bits.sh = t.bits;
+    BitSources src;
+    LaneCtx lc;
+    lc.direct = 0;
+    lc.cur = lc.next = kNoPos;
+    while (cur != kNoPos || split_at != kNoPos) {
         if (t.err) break;
-#ifndef GMK_POLL_MASK
-#define GMK_POLL_MASK 7u    // stop / watchdog / split / donation checks every 8 loop steps
-#endif
-        if ((++polls & GMK_POLL_MASK) == 0) {
+        if (split_at != kNoPos) {
+            if (sb && split_path(t, *sb, split_at)) break;
+            if (split_fail) { fail(t, o, split_fail); break; }
+            may_split = false;       // buffer full: finish this task here
+            split_at = kNoPos;
+        }
+        bool handed = false;         // the bit search's states went to the next round
+        if (bits_out) {
+            bits_out = false;
+            handed = sb && bits_split(t, *sb, bits);
+            if (!handed && split_fail) { fail(t, o, split_fail); break; }
+            if (!handed) may_split = false;
+            split_fail = 0;
+        }
+        // stop / watchdog / split / donation checks every 8 units: 1 a step, 4
+        // for a run of bit-search states, 8 for a block of children
+        polls += bits.active ? 4 : 1;
+        if (polls >= 8) {
+            polls = 0;
             int stop = 0, late = 0, hungry = 0, give = 0;
             if (t.lane == 0) {
                 stop = load_flag(o.stop) || (o.gstop && load_flag(o.gstop));
@@ -2007,64 +1768,149 @@ __device__ __forceinline__ unsigned long long run_dfs(Ctx& t, const Outputs& o, 
             stop = bcast(stop); late = bcast(late); hungry = bcast(hungry); give = bcast(give);
             if (stop) break;
             if (late) { fail(t, o, TASK_E_TIMEOUT); break; }
-            if (!kRec && give) donate_top(t, *db, cur, (unsigned long long)give);
+            if (!kRec && o.limit && t.cnt >= kFlushBatch) flush(t, o);
+            if (!kRec && give && !donate_top(t, *db, cur, (unsigned long long)give) && bits.active)
+                bits_donate(t, *db, bits);
             if (hungry) {
-                if (split_path(t, *sb, cur)) break;
-                may_split = false;   // buffer full: finish this task here
+                // the bit search's states first, then (at the next poll, which
+                // comes at once) the path
+                if (bits.active) bits_out = true;
+                else if (!handed) split_at = cur;
+                polls = 8;
+                if (!handed) continue;
             }
         }
         uint32_t* f = t.arena + cur;
-        const uint32_t flags = f[F_FLAGS];
         ChildReq req;
         bool want = false;
-        if (!(flags & FL_ENTERED)) {
-            if (t.lane == 0) f[F_FLAGS] = flags | FL_ENTERED;
-            __syncwarp();
-            t.nodes++;
-            task_nodes++;
-            const int r = enter_node<kRec, kBits>(t, o, cur, &req);
-            if (kRec && r == ENTER_DEFER) {
-                // re-enter this node next round, after the host drained the buffer
-                set_word(t, cur + F_FLAGS, flags);
-                t.nodes--;
-                task_nodes--;
-                if (sb && split_path(t, *sb, cur)) break;
-                fail(t, o, TASK_E_OUTBUF);
-                break;
+        if (!bits.active && !handed) {
+            const uint32_t flags = f[F_FLAGS];
+            bool start = false;
+            if (!(flags & FL_ENTERED)) {
+                if (t.lane == 0) f[F_FLAGS] = flags | FL_ENTERED;
+                __syncwarp();
+                t.nodes++;
+                task_nodes++;
+                const int r = enter_node<kRec, kBits>(t, o, cur, &req, bits, src);
+                if (kRec && r == ENTER_DEFER) {
+                    // re-enter this node next round, after the host drained the buffer
+                    set_word(t, cur + F_FLAGS, flags);
+                    t.nodes--;
+                    task_nodes--;
+                    split_at = cur;
+                    split_fail = TASK_E_OUTBUF;
+                    continue;
+                }
+                if (r == ENTER_DONE) {
+                    set_word(t, cur + F_PHASE, 2);
+                    if (!t.err) { cur = f[F_PARENT_SLOT]; continue; }
+                } else if (r == ENTER_BITS) {
+                    set_word(t, cur + F_PHASE, 2);
+                    start = true;
+                } else if (r == ENTER_PUSHED) {
+                    set_word(t, cur + F_PHASE, 2);   // the forced child is its only child
+                    want = true;
+                } else if ((flags & FL_ROOT) && f[F_ORDER] == 1u && (f[F_FLAGS] & FL_G1)) {
+                    const uint32_t p = f[F_POS];
+                    set_word(t, cur + F_POS, first > p ? first : p);
+                }
             }
-            if (r == ENTER_DONE) { set_word(t, cur + F_PHASE, 2); cur = f[F_PARENT_SLOT]; continue; }
-            if (r == ENTER_PUSHED) {
-                set_word(t, cur + F_PHASE, 2);   // the forced child is its only child
-                want = true;
-            } else if ((flags & FL_ROOT) && f[F_ORDER] == 1u && (f[F_FLAGS] & FL_G1)) {
-                const uint32_t p = f[F_POS];
-                set_word(t, cur + F_POS, first > p ? first : p);
+            if (!t.err && !start && lc.direct && lc.cur == cur) {
+                // the last block's children for the bit search, those that were
+                // not given away meanwhile
+                const Hdr h = read_hdr(f);
+                const int s = h.phase == 0 ? (int)h.order : 1 - (int)h.order;
+                const uint32_t pend = h.cnt.get(s);
+                lc.direct &= pend;
+                uint32_t rest = pend;
+                if (lc.direct) {
+                    const uint32_t bit = __ffs(lc.direct) - 1;
+                    lc.direct &= lc.direct - 1;
+                    pop_to(t, h.ns);
+                    if (lane_child(t, bits, src, h, s, h.phase == 1, bit)) {
+                        rest &= ~(1u << bit);
+                        t.nodes++;
+                        task_nodes++;
+                        start = true;
+                    }
+                }
+                if (t.lane == 0) {
+                    f[F_CNT0 + s] = rest;
+                    if (!lc.direct) f[F_FLAGS] |= FL_BUILD;   // the others are built
+                }
+                __syncwarp();
+                if (!start) continue;
             }
+            if (start) {
+                if (!bits_start(t, bits, src)) {
+                    if (!bits.lanes) cur = f[F_PARENT_SLOT];
+                    continue;
+                }
+            } else if (!t.err) {
+                if (!want) {
+                    Hdr h;
+                    const int nx = next_child(t, cur, lim.blocks, &req, &h);
+                    if (nx != NEXT_BLOCK) lc.cur = kNoPos;   // the lists are this frame's only
+                    if (nx == NEXT_NONE) { cur = f[F_PARENT_SLOT]; continue; }
+                    if (nx == NEXT_BLOCK) {
+                        uint32_t n = 0;
+                        lane_blocks<kRec>(t, o, cur, h, req.s, req.opp_done, lc, &n);
+                        t.nodes += n;
+                        task_nodes += n;
+                        polls = 8;
+                        continue;
+                    }
+                }
+                const uint32_t ch = build_child<kBits>(t, o, cur, req.c, req.s, req.p, req.forced, req.opp_done);
+                if (ch != kNoPos) { cur = ch; continue; }   // kNoPos: t.err is set
+            }
+            if (t.err == TASK_ARENA_FULL) {
+                // A node's scratch or a child did not fit.  Put the frame back
+                // as it was -- the node is entered again (its scratch, or a
+                // forced child: phase 2), or takes that child back -- and move
+                // the path to the next round, where each frame starts an empty
+                // arena.  Only a task's base frame that cannot hold its node or
+                // one child is an arena overflow (the split list's refusal
+                // reason 5 says so).
+                const uint32_t at = t.src[kSrcCap], site = t.src[kSrcCap + 1];
+                uint32_t* fa = t.arena + at;
+                const bool reenter = site == kSiteNode || fa[F_PHASE] == 2;
+                if (t.lane == 0) {
+                    const int s = fa[F_PHASE] == 0 ? (int)fa[F_ORDER] : 1 - (int)fa[F_ORDER];
+                    if (reenter) fa[F_FLAGS] &= ~FL_ENTERED;
+                    else if (lim.blocks && (fa[F_FLAGS] & gbit(s))) fa[F_CNT0 + s] |= 1u << (t.src[kSrcCap + 2] - fa[F_OFF0 + s]);
+                    else fa[F_POS] -= 1;
+                }
+                __syncwarp();
+                if (reenter) { t.nodes--; task_nodes--; }
+                t.err = 0;
+                if (at == 0) {
+                    if (sb && t.lane == 0) atomicCAS(sb->refused, 0, 5);
+                    fail(t, o, TASK_E_ARENA);
+                    break;
+                }
+                split_at = at;
+                split_fail = TASK_E_ARENA;
+                continue;
+            }
+            if (t.err) break;
         }
-        if (!want) want = next_child(t, cur, &req);
-        if (!want) { cur = f[F_PARENT_SLOT]; continue; }
-        const uint32_t ch = build_child<kBits>(t, o, cur, req.c, req.s, req.p, req.forced, req.opp_done);
-        cur = ch == kNoPos ? f[F_PARENT_SLOT] : ch;   // kNoPos: t.err is set, the loop ends
-    }
-    if (t.err == TASK_ARENA_FULL) {
-        // A node's scratch or a child did not fit.  Put the frame back as it
-        // was -- the node is entered again (its scratch, or a forced child:
-        // phase 2), or steps back one position in its phase -- and move the
-        // path to the next round, where each frame starts an empty arena.
-        // Only a task's base frame that cannot hold its node or one child is
-        // an arena overflow (the split list's refusal reason 5 says so).
-        const uint32_t at = t.src[kSrcCap], site = t.src[kSrcCap + 1];
-        uint32_t* f = t.arena + at;
-        const bool reenter = site == kSiteNode || f[F_PHASE] == 2;
-        if (t.lane == 0) {
-            if (reenter) f[F_FLAGS] &= ~FL_ENTERED;
-            else f[F_POS] -= 1;
+        // the bit search: a few states, or what it still has to hash
+        uint32_t n = 0;
+        if (!bits_run<kRec>(t, o, bits, &n)) {
+            // no room for a state's records: it goes to the next round, after
+            // the host drained the buffer
+            t.nodes--;
+            task_nodes--;
+            bits_out = true;
+            split_fail = TASK_E_OUTBUF;
         }
-        __syncwarp();
-        if (reenter) t.nodes--;
-        t.err = 0;
-        if (at == 0 && sb && t.lane == 0) atomicCAS(sb->refused, 0, 5);
-        if (!(at != 0 && sb && split_path(t, *sb, at))) fail(t, o, TASK_E_ARENA);
+        t.nodes += n;
+        task_nodes += n;
+        if (!bits.active) {
+            if (!bits.lanes) cur = f[F_PARENT_SLOT];
+            if (handed) polls = 8;   // the rest of the path follows: poll at once
+        }
     }
     pop_to(t, 0);
     return task_nodes;
@@ -2137,6 +1983,16 @@ __device__ __forceinline__ bool prep_record(Ctx& t, const Outputs& o, const uint
     h.off.b = F_WORDS + 2 * c0;
     h.top = F_WORDS + 2 * (c0 + c1);
     h.parent = kNoPos;
+    // a global side's pending children: ids of that side past its lower bound
+    #pragma unroll 1
+    for (int s = 0; s < 2; ++s) {
+        if (!(h.flags & gbit(s))) continue;
+        const uint32_t pend = __ldcg(fr + F_CNT0 + s), from = __ldcg(fr + F_OFF0 + s);
+        h.cnt.set(s, pend);
+        h.off.set(s, from);
+        bad |= pend && (from <= h.lo.get(s) || from >= side_end(t.g, s) ||
+                        side_end(t.g, s) - from < 32u - __clz(pend));
+    }
     const uint32_t* lr = fr + F_WORDS;
     #pragma unroll 1
     for (uint32_t i = t.lane; i < 2 * (c0 + c1); i += 32) {

@@ -13,6 +13,7 @@
 #include <algorithm>
 #include <chrono>
 #include <cmath>
+#include <cstddef>
 #include <cstdio>
 #include <cstring>
 #include <map>
@@ -54,8 +55,9 @@ struct Counters {
 // Per-round queue, split-buffer and record-buffer counters of the warp engine.
 struct RoundCounters {
     unsigned long long next_task, tasks_done, next_used, next_count, out_pos;
-    unsigned long long out_fail;    // lowest record position that found no room (~0: none)
-    unsigned long long next_fail;   // lowest split-record index that found no room (~0: none)
+    // complements, so that zeroed counters mean "none": of the lowest record
+    // position and of the lowest split-record index that found no room
+    unsigned long long out_fail, next_fail;
     int split_refused;              // first reason a split was refused (0 = none)
     int pad;
     // in-launch work sharing (gmk::warp::Donation); the polled counters sit on
@@ -65,7 +67,10 @@ struct RoundCounters {
     alignas(128) unsigned long long dq_tail;
     alignas(128) unsigned long long dq_claim;
     alignas(128) unsigned long long outstanding;
+    // the launch's work is done: one flag for every 32nd warp (not read back)
+    alignas(128) int done[gmk::warp::kDoneFlags][32];
 };
+constexpr size_t kRoundRead = offsetof(RoundCounters, done);   // bytes the host reads back
 
 constexpr int kBlock = 128;
 // Edge hash: at most this percentage of its slots hold keys (one per bucket of
@@ -131,29 +136,26 @@ enumerate_kernel(gmk::GraphView g, uint32_t k, Counters* ctr, uint32_t* arenas,
 }
 
 // One warp per block: warps are independent (no block-level sharing), and
-// single-warp blocks let the register file's last partial block count.  With
-// 25 resident blocks as the target, ptxas allocates 72 registers a thread (a
-// few spills) and 28 warps fit per SM; that measured 2-5 % faster on B200 than
-// 4-warp blocks at 80 registers (24 warps).  Among 4-warp blocks, 6 per SM (80
-// registers) was 6 % faster than 5 (96 registers, no spills) and 20 % faster
-// than 4; 7 and 8 (72 / 64 registers) lost to spills.
+// single-warp blocks let the register file's last partial block count.
 #ifndef GMK_WARP_BLOCK
 #define GMK_WARP_BLOCK 32                    // threads per block of the warp engine
 #endif
 constexpr int kWBlock = GMK_WARP_BLOCK;
 constexpr int kWarpsPerBlock = kWBlock / 32;
-// Resident blocks per SM the register allocation targets.
 #ifndef GMK_IDLE_SLEEP_MAX
-#define GMK_IDLE_SLEEP_MAX 1024u             // ns: longest back-off of a warp waiting for a record
+#define GMK_IDLE_SLEEP_MAX 256u              // ns: longest back-off of a warp waiting for a record
 #endif
-#ifndef GMK_WARP_MIN_BLOCKS
-#define GMK_WARP_MIN_BLOCKS 25
-#endif
-// The batch instantiation reads each task's graph from memory instead of the
-// kernel parameters, so it holds more live registers: at 72 it spilled 0.9 KB a
-// thread; 20 blocks (96 registers, 21 warps per SM) ran the mixed batch 7 %
-// faster than 25.
-constexpr int kBatchMinBlocks = 20;
+// Resident blocks per SM the register allocation targets.  The search is one
+// long kernel and each warp is at its own place in it, so more warps mean more
+// instruction-cache misses (28 warps at 72 registers: an issue slot in five
+// used, 19 of 36 stall cycles for instructions): 12 warps at 168 registers,
+// without spills, are faster almost everywhere (er200 k = 1 14.6 -> 10.9 ms, cl20k
+// first million 0.40 -> 0.23, cl100k k = 2 10.0 -> 7.7, cl500k k = 2 48.1 -> 41.6).
+// The exception is k = 1 over an edge hash far larger than L2 (cl500k, 537 MB),
+// whose probes wait for HBM: 28 warps 7.9 ms, 12 warps 10.0.
+constexpr int kWarpMinBlocks = 10;
+constexpr int kManyMinBlocks = 25;
+constexpr size_t kManyHashBytes = 256ull << 20;
 constexpr uint32_t kDefaultWarpArena = 1u << 18;
 // In-launch sharing: a task donates only after this many nodes of its own
 // (gmk_opts.donate_min_nodes 0).
@@ -201,7 +203,9 @@ struct WarpArgs {
     const uint32_t* cur_words;         // split records of the previous round
     const unsigned long long* cur_idx;
     gmk::warp::SplitBuf next;
-    uint32_t split_min_nodes;          // 0: never split
+    // 0: never split, and build children one by one (the plain schedule, which
+    // takes a root's tree in one warp, node by node)
+    uint32_t split_min_nodes;
     unsigned long long limit;
     uint32_t* out_buf;
     unsigned long long out_cap;
@@ -238,12 +242,16 @@ __device__ __forceinline__ const GraphTask& use_graph(const WarpArgs& a, uint32_
 }
 
 // kBatch: several graphs per launch; kRec: results written as records (the
-// count-only instantiation carries none of the record and drain code).
-template <bool kBatch, bool kRec, bool kBits>
-__global__ void __launch_bounds__(kWBlock, kBatch ? kBatchMinBlocks : GMK_WARP_MIN_BLOCKS)
+// count-only instantiation carries none of the record and drain code); kBits:
+// filter bitmaps for long lists (k >= 2); kMany: fewer registers, more warps.
+template <bool kBatch, bool kRec, bool kBits, bool kMany>
+__global__ void __launch_bounds__(kWBlock, kMany ? kManyMinBlocks : kWarpMinBlocks)
 enumerate_warp_kernel(const __grid_constant__ WarpArgs a) {
     __shared__ uint32_t s_sat[kWarpsPerBlock][gmk::kSatCap];
-    __shared__ uint32_t s_src[kWarpsPerBlock][gmk::warp::kSrcCap + 2];   // + arena-overflow note
+    __shared__ uint32_t s_src[kWarpsPerBlock][gmk::warp::kSrcCap + 3];   // + arena-overflow note
+    __shared__ gmk::warp::LaneShared s_lanes[kWarpsPerBlock];
+    // one of the two at a time: deciding a block, or a bit search
+    __shared__ union { gmk::warp::BitShared bits; gmk::warp::LaneScratch lanes; } s_part[kWarpsPerBlock];
     using namespace gmk::warp;
     const uint32_t wib = threadIdx.x >> 5;
     const uint32_t lane = lane_id();
@@ -275,9 +283,11 @@ enumerate_warp_kernel(const __grid_constant__ WarpArgs a) {
     t.scan_limit = a.pair_limit; t.err = 0;
     t.bits_min = a.bits_min_list;
     t.cnt = t.hsum = t.hxor = t.nodes = 0; t.work = 0;
-    t.sat = s_sat[wib]; t.src = s_src[wib]; t.lane = lane;
+    t.sat = s_sat[wib]; t.src = s_src[wib]; t.lanes = &s_lanes[wib];
+    t.bits = &s_part[wib].bits; t.lane_scratch = &s_part[wib].lanes; t.lane = lane;
     RunLimits lim;
     lim.split_min_nodes = a.split_min_nodes;
+    lim.blocks = a.split_min_nodes != 0;
     lim.queue = &a.rc->next_task;
     lim.queue_len = a.queue_len;
     lim.out_pos = &a.rc->out_pos;
@@ -286,6 +296,7 @@ enumerate_warp_kernel(const __grid_constant__ WarpArgs a) {
     // it, and so does any path that outgrows the arena (plain schedule too)
     const SplitBuf* sb = &a.next;
     const Donation* db = (!kRec && a.share.words) ? &a.share : nullptr;
+    unsigned long long left = 1;   // lane 0: tasks of the launch left after its last one
     for (;;) {
         unsigned long long j = ~0ull;
         int stop = 0;
@@ -310,6 +321,10 @@ enumerate_warp_kernel(const __grid_constant__ WarpArgs a) {
                 }
             }
         }
+        if (left == 0) {
+            for (uint32_t i = 0; i < kDoneFlags; ++i) *(volatile int*)(db->done + 32 * i) = 1;
+            left = 1;
+        }
         stop = bcast(stop);
         j = bcast(j);
         if (stop) break;
@@ -323,15 +338,17 @@ enumerate_warp_kernel(const __grid_constant__ WarpArgs a) {
             int quit = 0;
             if (lane == 0) {
                 const unsigned long long ticket = atomicAdd(db->claim, 1ull);
+                const volatile int* done = db->done + (wid % kDoneFlags) * 32;
                 unsigned long long seen = ~0ull, t_seen = gmk::now_ns();
-                unsigned sleep_ns = 64;
+                unsigned sleep_ns = 32;
                 for (uint32_t spin = 0;; ++spin) {
                     if (ticket < db->idx_cap) {
                         w = *(volatile unsigned long long*)(db->idx + ticket);
-                        if (w) break;
+                        if ((w ^ db->tag) >> kTagShift == 0) break;
                     }
-                    if ((spin & 7u) == 7u) {
-                        if (gmk::load_flag(o.stop)) { quit = 1; break; }
+                    if (*done) { quit = 1; break; }
+                    if ((spin & 7u) == 7u && gmk::load_flag(o.stop)) { quit = 1; break; }
+                    if ((spin & 63u) == 0) {
                         const unsigned long long out = *(volatile unsigned long long*)db->outstanding;
                         if (out + a.queue_len == 0) { quit = 1; break; }
                         // safety net: the work left must change (a task ends or a
@@ -357,16 +374,13 @@ enumerate_warp_kernel(const __grid_constant__ WarpArgs a) {
             quit = bcast(quit);
             if (quit) break;
             w = bcast(w);
-            rec = db->words + (w - 1);
+            rec = db->words + ((w & ((1ull << kTagShift) - 1)) - 1);
         } else {
             if (lane == 0) atomicAdd(&a.rc->tasks_done, 1ull);
             if (j < a.n_records) rec = a.cur_words + a.cur_idx[j];
         }
-        // Either kind of task writes its base frame, then enters the search.
-        // k = 1 kernels: one run_dfs call site for both kinds (the search loop
-        // is inlined once): 1.1-1.5x faster on complete runs than two inlined
-        // copies.  k >= 2 kernels (filter bitmaps): one copy per kind, which
-        // measured 1.1x faster there.
+        // Either kind of task writes its base frame, then enters the search (one
+        // run_dfs call site: the search loop is inlined once).
         uint32_t first = 0, attr = 0;
         bool go = false;
         unsigned long long* root_nodes = nullptr;
@@ -378,13 +392,6 @@ enumerate_warp_kernel(const __grid_constant__ WarpArgs a) {
             // a round that winds down hands its queued records on unchanged
             if (!(kRec && sb && draining(lim) && forward_record(t, *sb, rec)))
                 go = gmk::warp::prep_record(t, o, rec);
-            if constexpr (kBits) {
-                if (go) {
-                    const unsigned long long nodes = gmk::warp::run_dfs<kRec, kBits>(t, o, 0, sb, lim, db);
-                    if (root_nodes && lane == 0) atomicAdd(root_nodes + attr, nodes);
-                    go = false;
-                }
-            }
         } else {
             const unsigned long long id = a.root_task_base + (j - a.n_records);
             uint32_t root, last, gi = 0;
@@ -419,20 +426,19 @@ enumerate_warp_kernel(const __grid_constant__ WarpArgs a) {
             attr = root;
             if (!(kBatch && gmk::load_flag(o.gstop))) {   // a capped graph's tasks end at once
                 gmk::warp::prep_root(t, root, last);
-                if constexpr (kBits) {
-                    const unsigned long long nodes = gmk::warp::run_dfs<kRec, kBits>(t, o, first, sb, lim, db);
-                    if (root_nodes && lane == 0) atomicAdd(root_nodes + attr, nodes);
-                } else {
-                    go = true;
-                }
+                go = true;
             }
         }
-        if (!kBits && go) {
+        if (go) {
             const unsigned long long nodes = gmk::warp::run_dfs<kRec, kBits>(t, o, first, sb, lim, db);
             if (root_nodes && lane == 0) atomicAdd(root_nodes + attr, nodes);
         }
-        if (db && lane == 0) atomicAdd(db->outstanding, ~0ull);   // this task is finished
-        flush(t, o);
+        // this task is finished; the last one of the launch ends the waiting
+        if (db && lane == 0) left = atomicAdd(db->outstanding, ~0ull) - 1 + a.queue_len;
+        // counts go out per task where they may stop the run or change owner;
+        // five atomics on one line per task would cost short tasks more than
+        // their search
+        if (kBatch || o.limit) flush(t, o);
         if (t.err) break;
     }
     flush(t, o);
@@ -485,6 +491,7 @@ enumerate_dense_kernel(const __grid_constant__ DenseArgs a) {
     uint32_t gid = 0xFFFFFFFFu;
     unsigned long long limit = a.limit;
     Counters* ctr = nullptr;
+    unsigned long long left = 1;   // lane 0: tasks of the launch left after its last one
     // results and nodes of the current graph so far to its counters
     auto flush = [&]() {
         if (t.nfound) flush_found<N>(t);
@@ -508,6 +515,10 @@ enumerate_dense_kernel(const __grid_constant__ DenseArgs a) {
             stop = gmk::load_flag(&a.ctr->stop);
             if (!stop) j = atomicAdd(&a.rc->next_task, 1ull);
         }
+        if (left == 0) {
+            for (uint32_t i = 0; i < gmk::warp::kDoneFlags; ++i) *(volatile int*)(a.share.done + 32 * i) = 1;
+            left = 1;
+        }
         stop = bcast(stop);
         j = bcast(j);
         if (stop) break;
@@ -523,12 +534,14 @@ enumerate_dense_kernel(const __grid_constant__ DenseArgs a) {
             if (lane == 0) {
                 ticket = atomicAdd(a.share.claim, 1ull);
                 const volatile uint32_t* slot = a.share.rec + ticket * kRecordWords;
+                const volatile int* done = a.share.done + (blockIdx.x % gmk::warp::kDoneFlags) * 32;
                 unsigned long long seen = ~0ull, t_seen = gmk::now_ns();
                 unsigned sleep_ns = 32;
                 for (uint32_t spin = 0;; ++spin) {
                     if (ticket < a.share.slots && *slot == a.share.launch) break;
-                    if ((spin & 7u) == 7u) {
-                        if (gmk::load_flag(&a.ctr->stop)) { quit = 1; break; }
+                    if (*done) { quit = 1; break; }
+                    if ((spin & 7u) == 7u && gmk::load_flag(&a.ctr->stop)) { quit = 1; break; }
+                    if ((spin & 63u) == 0) {
                         const unsigned long long out = *(volatile unsigned long long*)a.share.outstanding;
                         if (out + a.queue_len == 0) { quit = 1; break; }
                         // safety net: the work left must change within the limit
@@ -608,7 +621,7 @@ enumerate_dense_kernel(const __grid_constant__ DenseArgs a) {
         #pragma unroll
         for (int w = N - 1; w >= 0; --w)
             if (s.iu[w]) root = 32 * w + __ffs(s.iu[w]) - 1;
-        t.sp = t.bottom = 0;
+        t.sp = t.bottom = t.extra = 0;
         uint32_t polls = 0;
         unsigned long long nodes = 0;
         bool quit = kBatch && gmk::load_flag(&ctr->stop);   // a capped graph's tasks end at once
@@ -651,7 +664,10 @@ enumerate_dense_kernel(const __grid_constant__ DenseArgs a) {
                 if (limit && t.cnt >= gmk::kFlushBatch) flush();
             }
             ++nodes;
-            if (!node<N>(t, s)) {
+            const bool down = node<N>(t, s);
+            nodes += t.extra;
+            t.extra = 0;
+            if (!down) {
                 if (t.sp == t.bottom) {
                     have = false;
                 } else {
@@ -665,10 +681,27 @@ enumerate_dense_kernel(const __grid_constant__ DenseArgs a) {
         t.nodes += nodes;
         if (lane == 0) {
             if (G.root_nodes) atomicAdd(G.root_nodes + root, nodes);
-            if (share) atomicAdd(a.share.outstanding, ~0ull);   // this task is finished
+            // this task is finished; the last one of the launch ends the waiting
+            if (share) left = atomicAdd(a.share.outstanding, ~0ull) - 1 + a.queue_len;
         }
     }
     flush();
+}
+
+// The instantiations of the list-based kernel.
+enum WarpKernel : int { kWarpCount, kWarpCountBits, kWarpCountMany, kWarpRec, kWarpRecBits, kWarpRecMany, kWarpBatch };
+constexpr int kWarpKernels = 7;
+typedef void (*WarpKernelFn)(const WarpArgs);
+WarpKernelFn warp_kernel(int which) {
+    switch (which) {
+        case kWarpCount: return enumerate_warp_kernel<false, false, false, false>;
+        case kWarpCountBits: return enumerate_warp_kernel<false, false, true, false>;
+        case kWarpCountMany: return enumerate_warp_kernel<false, false, false, true>;
+        case kWarpRec: return enumerate_warp_kernel<false, true, false, false>;
+        case kWarpRecBits: return enumerate_warp_kernel<false, true, true, false>;
+        case kWarpRecMany: return enumerate_warp_kernel<false, true, false, true>;
+        default: return enumerate_warp_kernel<true, false, false, false>;
+    }
 }
 
 // CSR check on the device: thread i checks vertex i (offsets non-decreasing
@@ -788,13 +821,13 @@ struct Workspace {
     size_t split_words_bytes[2] = {0, 0};
     unsigned long long* d_split_idx[2] = {nullptr, nullptr};
     size_t split_idx_bytes[2] = {0, 0};
-    // in-launch work sharing: donated records and their slot index (slots the
-    // last launch may have written are cleared before the next one)
+    // in-launch work sharing: donated records and their slot index (a slot is
+    // valid for the launch whose number it carries)
     uint32_t* d_dq_words = nullptr;
     size_t dq_words_bytes = 0;
     unsigned long long* d_dq_idx = nullptr;
     size_t dq_idx_bytes = 0;
-    unsigned long long dq_dirty = 0;
+    uint32_t dq_launch = 0;       // the last launch's number; 0: the index is not cleared yet
     // small graphs' search: stack spill, records of shared states (each valid for
     // the launch whose number it carries), counters of a launch and their pinned
     // copy on the host
@@ -819,7 +852,8 @@ Workspace g_ws[kMaxDevices];
 // Per-device launch facts, looked up once (under the workspace mutex).
 struct DeviceInfo {
     bool ready = false;
-    int sms = 0, per_sm_warp = 0, per_sm_batch = 0, per_sm_thread = 0;
+    int sms = 0, per_sm_thread = 0;
+    int per_sm_warp[7] = {};              // [WarpKernel]
     int per_sm_dense[5][2] = {};   // [N = 1..4][one graph, batch]
 };
 DeviceInfo g_dev[kMaxDevices];
@@ -1194,18 +1228,25 @@ std::vector<uint32_t> select_roots(uint32_t nl, const float* cost, uint32_t rb, 
     return std::vector<uint32_t>(order.begin() + rb, order.begin() + re);
 }
 
+// Narrowest chunk of first-level children: of gmk_plan_tasks, and of the
+// tasks that a run of the list-based kernel makes itself -- its children are
+// looked at 32 at a time.
+constexpr uint32_t kPlanChunk = 16;
+constexpr uint32_t kMinChunk = 64;
+
 // Splits each root into m chunks of its first-level V children in proportion
-// to its cost (m = ceil(cost / unit), at most max_chunks, chunks at least 16
-// children wide) and appends them with per-task cost cost / m and graph
+// to its cost (m = ceil(cost / unit), at most max_chunks, chunks at least
+// min_width children wide) and appends them with per-task cost cost / m and graph
 // index gi, largest per-task cost first, ties in `roots` order.  That is the
 // order a stable sort of the tasks by cost gives (a root's chunks share one
 // cost and stay together), at the price of sorting the roots only: for the
 // headline graph 623 roots instead of 24 k tasks.
 void chunk_roots(uint32_t nl, uint32_t n, const std::vector<uint32_t>& roots, const float* cost,
-                 double unit, uint32_t max_chunks, uint32_t gi, std::vector<gmk_task>& out) {
+                 double unit, uint32_t max_chunks, uint32_t min_width, uint32_t gi,
+                std::vector<gmk_task>& out) {
     const uint32_t nv = n - nl;
     if (!nv) return;
-    const uint32_t wide = std::max<uint32_t>(1, nv / 16);
+    const uint32_t wide = std::max<uint32_t>(1, nv / min_width);
     struct RootChunks { uint32_t r, m; float c; };
     std::vector<RootChunks> rc;
     rc.reserve(roots.size());
@@ -1275,7 +1316,7 @@ bool is_planned(const std::vector<GraphJob>& jobs, const gmk_opts* opts) {
 
 // The planned tasks of a run for `workers` workers, at most max_chunks a root.
 int plan_jobs(std::vector<GraphJob>& jobs, const gmk_opts* opts, uint64_t workers,
-              uint32_t max_chunks, std::vector<gmk_task>& plan) {
+              uint32_t max_chunks, uint32_t min_width, std::vector<gmk_task>& plan) {
     int rc;
     const size_t ng = jobs.size();
     const uint32_t nsh = opts->nshards > 1 ? opts->nshards : 1u;
@@ -1299,7 +1340,7 @@ int plan_jobs(std::vector<GraphJob>& jobs, const gmk_opts* opts, uint64_t worker
     }
     const double unit = total / (double)std::max<uint64_t>(1, (uint64_t)tasks_per * workers);
     for (size_t i = 0; i < ng; ++i)
-        chunk_roots(jobs[i].g->nl, jobs[i].g->n, roots[i], costs[i], unit, max_chunks,
+        chunk_roots(jobs[i].g->nl, jobs[i].g->n, roots[i], costs[i], unit, max_chunks, min_width,
                     (uint32_t)i, plan);
     order_and_shard(plan, nsh, sh, ng == 1);
     // Under a result limit (the run's, or a batch graph's cap) balance does
@@ -1422,7 +1463,7 @@ int run_dense(std::vector<GraphJob>& jobs, const gmk_opts* opts, int words, Work
     const bool planned = is_planned(jobs, opts);
     const uint32_t max_chunks = opts->schedule == GMK_SCHEDULE_PLAIN ? 1u : 0xFFFFFFFFu;
     if (planned) {
-        if ((rc = plan_jobs(jobs, opts, workers, max_chunks, plan))) return rc;
+        if ((rc = plan_jobs(jobs, opts, workers, max_chunks, kPlanChunk, plan))) return rc;
         if ((rc = upload_plan(ws, g0, plan))) return rc;
     }
     const size_t ctr_bytes = sizeof(DenseCounters) + (ng > 1 ? (ng - 1) * sizeof(Counters) : 0);
@@ -1493,6 +1534,7 @@ int run_dense(std::vector<GraphJob>& jobs, const gmk_opts* opts, int words, Work
         a.share.outstanding = &dc->rc.outstanding;
         a.share.donated = &dc->rc.donated;
         a.share.full = &dc->rc.dq_full;
+        a.share.done = &dc->rc.done[0][0];
         a.share.min_nodes = opts->donate_min_nodes ? opts->donate_min_nodes : kDenseDonateMin;
     }
     a.single = gt[0];
@@ -1561,10 +1603,8 @@ int run_jobs(std::vector<GraphJob>& jobs, const gmk_opts* opts, gmk_sink sink, v
     if (!di.ready) {
         int sms = 0;
         CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &di.per_sm_warp, enumerate_warp_kernel<false, false, false>, kWBlock, 0));
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &di.per_sm_batch, enumerate_warp_kernel<true, false, false>, kWBlock, 0));
+        for (int i = 0; i < kWarpKernels; ++i)
+            CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&di.per_sm_warp[i], warp_kernel(i), kWBlock, 0));
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&di.per_sm_thread, enumerate_kernel,
                                                          kBlock, 0));
         if (int rc = dense_occupancy<1>(di)) return rc;
@@ -1575,8 +1615,14 @@ int run_jobs(std::vector<GraphJob>& jobs, const gmk_opts* opts, gmk_sink sink, v
         di.ready = true;
     }
     if (const int words = dense_words(jobs, opts)) return run_dense(jobs, opts, words, ws, di, outs);
-    // resident blocks per SM of the instantiation this run launches
-    const int per_sm = std::max(!warp ? di.per_sm_thread : jobs.size() > 1 ? di.per_sm_batch : di.per_sm_warp, 1);
+    // the instantiation this run launches (k >= 2: with filter bitmaps for long
+    // lists; a batch has no records), its resident blocks per SM
+    const bool bits = jobs[0].k >= 2;
+    const int which = jobs.size() > 1 ? kWarpBatch
+                      : bits          ? (opts->emit ? kWarpRecBits : kWarpCountBits)
+                      : g0->eh_bytes > kManyHashBytes ? (opts->emit ? kWarpRecMany : kWarpCountMany)
+                                                      : (opts->emit ? kWarpRec : kWarpCount);
+    const int per_sm = std::max(warp ? di.per_sm_warp[which] : di.per_sm_thread, 1);
     const int block = warp ? kWBlock : kBlock;
     const uint32_t lanes_per_worker = warp ? 32u : 1u;
     uint32_t max_degree = 0, max_k = 1;
@@ -1639,7 +1685,7 @@ int run_jobs(std::vector<GraphJob>& jobs, const gmk_opts* opts, gmk_sink sink, v
     const bool planned = is_planned(jobs, opts);
     std::vector<gmk_task> plan;
     const uint32_t max_chunks = opts->schedule == GMK_SCHEDULE_PLAIN ? 1u : 0xFFFFFFFFu;
-    if (planned && (rc = plan_jobs(jobs, opts, workers, max_chunks, plan))) return rc;
+    if (planned && (rc = plan_jobs(jobs, opts, workers, max_chunks, kMinChunk, plan))) return rc;
     unsigned long long n_tasks = 0;
     for (size_t i = 0; i < ng; ++i) {
         const GraphJob& j = jobs[i];
@@ -1651,10 +1697,10 @@ int run_jobs(std::vector<GraphJob>& jobs, const gmk_opts* opts, gmk_sink sink, v
             if (opts->chunk) {
                 chunk = std::min(opts->chunk, nv);
             } else {
-                // about tasks_per (8) tasks per worker, but no chunk below 16 children
+                // about tasks_per (8) tasks per worker, but no chunk below kMinChunk children
                 const uint64_t want = (uint64_t)tasks_per * workers;
                 const uint64_t per_root = (want + g->nl - 1) / std::max<uint32_t>(g->nl, 1);
-                chunk = (uint32_t)std::max<uint64_t>(16, (nv + per_root - 1) / std::max<uint64_t>(1, per_root));
+                chunk = (uint32_t)std::max<uint64_t>(kMinChunk, (nv + per_root - 1) / std::max<uint64_t>(1, per_root));
                 chunk = std::min(chunk, nv);
             }
         }
@@ -1727,7 +1773,7 @@ int run_jobs(std::vector<GraphJob>& jobs, const gmk_opts* opts, gmk_sink sink, v
         const void* had_p = ws.d_dq_idx;
         if ((rc = grow((void**)&ws.d_dq_words, &ws.dq_words_bytes, dq_word_cap * 4))) return rc;
         if ((rc = grow((void**)&ws.d_dq_idx, &ws.dq_idx_bytes, dq_idx_cap * 8))) return rc;
-        if (ws.dq_idx_bytes != had || ws.d_dq_idx != had_p) ws.dq_dirty = ws.dq_idx_bytes / 8;
+        if (ws.dq_idx_bytes != had || ws.d_dq_idx != had_p) ws.dq_launch = 0;
     }
     const unsigned grid = (unsigned)(threads / block);
     const unsigned long long watchdog_ns = (unsigned long long)opts->watchdog_ms * 1000000ull;
@@ -1791,6 +1837,7 @@ int run_jobs(std::vector<GraphJob>& jobs, const gmk_opts* opts, gmk_sink sink, v
             a.share.outstanding = &rcd->outstanding;
             a.share.donated = &rcd->donated;
             a.share.full = &rcd->dq_full;
+            a.share.done = &rcd->done[0][0];
             a.share.min_nodes = opts->donate_min_nodes ? opts->donate_min_nodes : kDefaultDonateMin;
         }
         // Record mode streams: each round writes one of two record buffers,
@@ -1820,47 +1867,36 @@ int run_jobs(std::vector<GraphJob>& jobs, const gmk_opts* opts, gmk_sink sink, v
             a.next.idx_cap = split_idx_cap;
             a.out_buf = opts->emit ? outb[round & 1] : nullptr;
             CK(cudaMemsetAsync(g0->d_rc, 0, sizeof(RoundCounters), g0->stream));
-            CK(cudaMemsetAsync(&g0->d_rc->out_fail, 0xFF, 2 * sizeof(unsigned long long), g0->stream));
-            if (share && ws.dq_dirty) {
-                // every slot an earlier launch may have written, not only this one's
-                CK(cudaMemsetAsync(ws.d_dq_idx, 0,
-                                   8ull * std::min<unsigned long long>(ws.dq_dirty, ws.dq_idx_bytes / 8),
-                                   g0->stream));
-                ws.dq_dirty = 0;
+            if (share) {
+                // a slot counts when it carries this launch's number: a new
+                // index, and one whose numbers are used up, starts cleared
+                if (ws.dq_launch == 0 || ++ws.dq_launch >= 1u << (64 - gmk::warp::kTagShift)) {
+                    CK(cudaMemsetAsync(ws.d_dq_idx, 0, ws.dq_idx_bytes, g0->stream));
+                    ws.dq_launch = 1;
+                }
+                a.share.tag = (unsigned long long)ws.dq_launch << gmk::warp::kTagShift;
             }
-            // k >= 2: the instantiation with filter bitmaps for long lists
-            // (at k = 1 their code alone cost 15 %, so it is a separate kernel)
-            const bool bits = a.single.k >= 2;
-            if (ng == 1 && !opts->emit && !bits)
-                enumerate_warp_kernel<false, false, false><<<grid, kWBlock, 0, g0->stream>>>(a);
-            else if (ng == 1 && !opts->emit)
-                enumerate_warp_kernel<false, false, true><<<grid, kWBlock, 0, g0->stream>>>(a);
-            else if (ng == 1 && !bits)
-                enumerate_warp_kernel<false, true, false><<<grid, kWBlock, 0, g0->stream>>>(a);
-            else if (ng == 1)
-                enumerate_warp_kernel<false, true, true><<<grid, kWBlock, 0, g0->stream>>>(a);
-            else   // a batch has no records
-                enumerate_warp_kernel<true, false, false><<<grid, kWBlock, 0, g0->stream>>>(a);
+            warp_kernel(which)<<<grid, kWBlock, 0, g0->stream>>>(a);
             CK(cudaGetLastError());
+            CK(cudaEventRecord(g0->ev1, g0->stream));   // the last round's stands
             if (pending >= 0 && sink_rc == GMK_OK) {
                 sink_rc = deliver_records(g0, outb[pending], pending_words, sink, user);
                 pending = -1;
             }
             RoundCounters r;
-            CK(cudaMemcpyAsync(&r, g0->d_rc, sizeof(r), cudaMemcpyDeviceToHost, g0->stream));
+            CK(cudaMemcpyAsync(&r, g0->d_rc, kRoundRead, cudaMemcpyDeviceToHost, g0->stream));
             CK(cudaMemcpyAsync(&h, launch_ctr, sizeof(h), cudaMemcpyDeviceToHost, g0->stream));
             CK(cudaStreamSynchronize(g0->stream));
             ++rounds;
             tasks_total += a.queue_len;
             tasks_done += std::min<unsigned long long>(r.tasks_done, a.queue_len);
             if (share) {
-                ws.dq_dirty = std::max<unsigned long long>(ws.dq_dirty, std::min(r.dq_tail, dq_idx_cap));
                 donations += r.donated;
             }
             if (opts->emit) {
                 // records end where the first one found no room
                 pending = round & 1;
-                pending_words = std::min({r.out_pos, (unsigned long long)out_words, r.out_fail});
+                pending_words = std::min({r.out_pos, (unsigned long long)out_words, ~r.out_fail});
             }
             const unsigned long long consumed = std::min(r.next_task, a.queue_len);
             if (consumed > n_records) root_next += consumed - n_records;
@@ -1873,7 +1909,7 @@ int run_jobs(std::vector<GraphJob>& jobs, const gmk_opts* opts, gmk_sink sink, v
                              why[r.split_refused >= 0 && r.split_refused <= 5 ? r.split_refused : 0];
             }
             if (h.error || h.stop || sink_rc != GMK_OK) break;
-            const unsigned long long next = std::min({r.next_count, split_idx_cap, r.next_fail});
+            const unsigned long long next = std::min({r.next_count, split_idx_cap, ~r.next_fail});
             if (next == 0 && root_next >= my_tasks) break;
             if (watchdog_ns) {
                 const double el = std::chrono::duration<double>(std::chrono::steady_clock::now() -
@@ -1883,8 +1919,6 @@ int run_jobs(std::vector<GraphJob>& jobs, const gmk_opts* opts, gmk_sink sink, v
             n_records = next;
             cur ^= 1;
         }
-        CK(cudaEventRecord(g0->ev1, g0->stream));
-        CK(cudaStreamSynchronize(g0->stream));
         if (pending >= 0 && sink_rc == GMK_OK && !h.error)
             sink_rc = deliver_records(g0, outb[pending], pending_words, sink, user);
         if (sink_rc < 0 && sink_rc != GMK_E_SINK) return sink_rc;
@@ -1962,7 +1996,7 @@ int gmk_plan_tasks(uint32_t n, uint32_t n_left, const float* root_cost, uint32_t
     for (const uint32_t r : roots) total += std::max<double>(root_cost[r], 0.0);
     std::vector<gmk_task> plan;
     chunk_roots(n_left, n, roots, root_cost, total / (double)std::max<uint64_t>(1, target_tasks),
-                max_chunks ? max_chunks : 0xFFFFFFFFu, 0, plan);
+                max_chunks ? max_chunks : 0xFFFFFFFFu, kPlanChunk, 0, plan);
     order_and_shard(plan, nshards, shard, true);
     if (out) std::copy(plan.begin(), plan.end(), out);
     *n_out = plan.size();
