@@ -2085,7 +2085,7 @@ struct gmk_mlp {
     __half* d_x = nullptr;
     float* d_xf = nullptr;
     float* d_y = nullptr;
-    float* d_act = nullptr;
+    float* d_part = nullptr;     // per-block gradient sums
     float* d_out = nullptr;
     uint32_t cap = 0;
 };
@@ -2096,14 +2096,13 @@ using gmk::mlp::NP;
 
 int mlp_reserve(gmk_mlp* m, uint32_t n) {
     if (n <= m->cap) return GMK_OK;
-    cudaFree(m->d_x); cudaFree(m->d_xf); cudaFree(m->d_y); cudaFree(m->d_act); cudaFree(m->d_out);
-    m->d_x = nullptr; m->d_xf = nullptr; m->d_y = nullptr; m->d_act = nullptr; m->d_out = nullptr;
+    cudaFree(m->d_x); cudaFree(m->d_xf); cudaFree(m->d_y); cudaFree(m->d_out);
+    m->d_x = nullptr; m->d_xf = nullptr; m->d_y = nullptr; m->d_out = nullptr;
     m->cap = 0;
     const uint64_t nn = n;
     CK(cudaMalloc(&m->d_x, nn * gmk::mlp::F * sizeof(__half)));
     CK(cudaMalloc(&m->d_xf, nn * gmk::mlp::F * sizeof(float)));
     CK(cudaMalloc(&m->d_y, nn * sizeof(float)));
-    CK(cudaMalloc(&m->d_act, nn * 2 * gmk::mlp::H * sizeof(float)));
     CK(cudaMalloc(&m->d_out, nn * sizeof(float)));
     m->cap = n;
     return GMK_OK;
@@ -2120,15 +2119,31 @@ int mlp_upload(gmk_mlp* m, const float* x, const float* y, uint32_t n) {
     return GMK_OK;
 }
 
+constexpr size_t kForwardShared = sizeof(gmk::mlp::TileShared);
+constexpr size_t kGradientShared = (sizeof(gmk::mlp::TileShared) + 15) / 16 * 16 + sizeof(gmk::mlp::TileGrad);
+constexpr uint32_t kModelBlocks = 148;   // one block (of tiles) per SM
+
+// Predictions of n FP16 samples into out (device).
+int mlp_forward(const gmk_mlp* m, const __half* x, uint32_t n, float* out, cudaStream_t s) {
+    const uint32_t tiles = (n + gmk::mlp::kTile - 1) / gmk::mlp::kTile;
+    CK(cudaFuncSetAttribute(gmk::mlp::forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            (int)kForwardShared));
+    gmk::mlp::forward_kernel<<<std::min(tiles, 2 * kModelBlocks), gmk::mlp::kThreads, kForwardShared, s>>>(
+        m->d_w, x, n, out);
+    CK(cudaGetLastError());
+    return GMK_OK;
+}
+
 // Forward + backward of the MSE over n uploaded samples into d_grad / d_loss.
 int mlp_grad(gmk_mlp* m, uint32_t n) {
-    CK(cudaMemset(m->d_grad, 0, NP * sizeof(float)));
-    CK(cudaMemset(m->d_loss, 0, sizeof(float)));
-    const unsigned grid = (n + gmk::mlp::kBlock - 1) / gmk::mlp::kBlock;
-    gmk::mlp::forward_kernel<<<grid, gmk::mlp::kBlock>>>(m->d_w, m->d_x, n, m->d_act, m->d_out);
+    if (!m->d_part) CK(cudaMalloc(&m->d_part, sizeof(float) * (NP + 1) * kModelBlocks));
+    const uint32_t blocks = std::min((n + gmk::mlp::kTile - 1) / gmk::mlp::kTile, kModelBlocks);
+    CK(cudaFuncSetAttribute(gmk::mlp::gradient_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            (int)kGradientShared));
+    gmk::mlp::gradient_kernel<<<blocks, gmk::mlp::kThreads, kGradientShared>>>(m->d_w, m->d_x, m->d_y, n,
+                                                                              m->d_part);
     CK(cudaGetLastError());
-    gmk::mlp::backward_kernel<<<grid, gmk::mlp::kBlock>>>(m->d_w, m->d_x, m->d_y, m->d_act,
-                                                         m->d_out, n, m->d_grad, m->d_loss);
+    gmk::mlp::gradient_sum_kernel<<<(4 * (NP + 1) + 255) / 256, 256>>>(m->d_part, blocks, m->d_grad, m->d_loss);
     CK(cudaGetLastError());
     return GMK_OK;
 }
@@ -2198,7 +2213,7 @@ void gmk_mlp_free(gmk_mlp* m) {
     cudaSetDevice(m->device);
     cudaFree(m->d_master); cudaFree(m->d_w); cudaFree(m->d_m); cudaFree(m->d_v);
     cudaFree(m->d_grad); cudaFree(m->d_loss);
-    cudaFree(m->d_x); cudaFree(m->d_xf); cudaFree(m->d_y); cudaFree(m->d_act); cudaFree(m->d_out);
+    cudaFree(m->d_x); cudaFree(m->d_xf); cudaFree(m->d_y); cudaFree(m->d_part); cudaFree(m->d_out);
     delete m;
 }
 
@@ -2266,10 +2281,7 @@ int gmk_mlp_predict_roots(gmk_mlp* m, const gmk_graph* g, uint32_t k, float* out
     gmk::mlp::root_features_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, g->stream>>>(
         gv, k, gm->d_feat);
     CK(cudaGetLastError());
-    const unsigned grid = (g->nl + gmk::mlp::kBlock - 1) / gmk::mlp::kBlock;
-    gmk::mlp::forward_kernel<<<grid, gmk::mlp::kBlock, 0, g->stream>>>(m->d_w, gm->d_feat, g->nl,
-                                                                      nullptr, m->d_out);
-    CK(cudaGetLastError());
+    if (int rc = mlp_forward(m, gm->d_feat, g->nl, m->d_out, g->stream)) return rc;
     CK(cudaMemcpyAsync(out, m->d_out, 4ull * g->nl, cudaMemcpyDeviceToHost, g->stream));
     CK(cudaStreamSynchronize(g->stream));
     return GMK_OK;
@@ -2280,9 +2292,7 @@ int gmk_mlp_predict(gmk_mlp* m, const float* x, uint32_t n, float* out) {
     if (n == 0) return GMK_OK;
     CK(cudaSetDevice(m->device));
     if (int rc = mlp_upload(m, x, nullptr, n)) return rc;
-    const unsigned grid = (n + gmk::mlp::kBlock - 1) / gmk::mlp::kBlock;
-    gmk::mlp::forward_kernel<<<grid, gmk::mlp::kBlock>>>(m->d_w, m->d_x, n, nullptr, m->d_out);
-    CK(cudaGetLastError());
+    if (int rc = mlp_forward(m, m->d_x, n, m->d_out, nullptr)) return rc;
     CK(cudaMemcpy(out, m->d_out, (uint64_t)n * sizeof(float), cudaMemcpyDeviceToHost));
     return GMK_OK;
 }

@@ -1,6 +1,6 @@
 // Subtree-size model for the learned schedule: a 16-64-64-1 perceptron with
 // ReLU hidden layers, FP16 weights and inputs, FP32 accumulation, trained on
-// the GPU by the kernels below (forward, backward, Adam).  Target: log1p of a
+// the GPU by the kernels below (forward, gradient, Adam).  Target: log1p of a
 // root task's search-tree nodes.  The model only orders the roots (largest
 // predicted first); it never prunes, so the result set does not depend on it.
 //
@@ -31,7 +31,6 @@ constexpr int OFF_B2 = OFF_W2 + H * H;
 constexpr int OFF_W3 = OFF_B2 + H;
 constexpr int OFF_B3 = OFF_W3 + H;
 constexpr int NP = OFF_B3 + 1;   // 5313 parameters
-constexpr int kBlock = 128;
 
 // One warp per root: the 16 features of root task x.
 __global__ void root_features_kernel(GraphView g, uint32_t k, __half* out) {
@@ -85,85 +84,249 @@ __global__ void root_features_kernel(GraphView g, uint32_t k, __half* out) {
     for (int i = 0; i < F; ++i) out[x * F + i] = __float2half_rn(log1pf(f[i]));
 }
 
-__device__ __forceinline__ void stage_weights(const __half* w, __half* sw) {
-    for (int i = threadIdx.x; i < NP; i += blockDim.x) sw[i] = w[i];
+// Samples go through the model in tiles of kTile, one tile per block at a time;
+// the block's 16 x 16 threads each own 4 x 4 outputs of every 64 x 64 product
+// (FP32 multiply-adds in the order of a plain loop over k).  Operands are in
+// shared memory with k as the slow index, so that a k step reads one float4 per
+// operand and thread.  Rows are padded by 4 words: a transposed store then
+// spreads over the banks, and float4 reads stay aligned.
+constexpr int kTile = 64;
+constexpr int kThreads = 256;
+constexpr int kPitch = kTile + 4;
+
+struct TileShared {
+    float w1t[F][kPitch];        // W1 transposed: [f][j]
+    float w2t[H][kPitch];        // W2 transposed: [q][j]
+    float b1[H], b2[H], w3[H];
+    float xt[F][kPitch];         // [f][sample]
+    float h1t[H][kPitch];        // [q][sample]
+    float h2t[H][kPitch];        // [j][sample]; the backward pass: dh2 likewise
+    float out[kTile];
+    float b3;
+};
+// What only the backward pass keeps.
+struct TileGrad {
+    float w2[H][kPitch];         // [j][q]
+    float x[kTile][F + 4];       // [sample][f]
+    float h1[kTile][kPitch];     // [sample][q]; later dh1
+    float dh2[kTile][kPitch];    // [sample][j]
+    float dout[kTile];
+    float red[kThreads];
+};
+
+__device__ __forceinline__ void load_weights(const __half* w, TileShared& s) {
+    for (int i = threadIdx.x; i < H * F; i += kThreads) s.w1t[i % F][i / F] = __half2float(w[OFF_W1 + i]);
+    for (int i = threadIdx.x; i < H * H; i += kThreads) s.w2t[i % H][i / H] = __half2float(w[OFF_W2 + i]);
+    for (int i = threadIdx.x; i < H; i += kThreads) {
+        s.b1[i] = __half2float(w[OFF_B1 + i]);
+        s.b2[i] = __half2float(w[OFF_B2 + i]);
+        s.w3[i] = __half2float(w[OFF_W3 + i]);
+    }
+    if (threadIdx.x == 0) s.b3 = __half2float(w[OFF_B3]);
+}
+
+// acc[a][b] += sum over k of left[k][4 ty + a] * right[k][4 tx + b]
+template <int K, int PL, int PR>
+__device__ __forceinline__ void product(const float (*left)[PL], const float (*right)[PR], int ty, int tx,
+                                        float (&acc)[4][4]) {
+    #pragma unroll 8
+    for (int k = 0; k < K; ++k) {
+        const float4 l = *reinterpret_cast<const float4*>(&left[k][4 * ty]);
+        const float4 r = *reinterpret_cast<const float4*>(&right[k][4 * tx]);
+        const float la[4] = {l.x, l.y, l.z, l.w}, ra[4] = {r.x, r.y, r.z, r.w};
+        #pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            #pragma unroll
+            for (int b = 0; b < 4; ++b) acc[a][b] = fmaf(la[a], ra[b], acc[a][b]);
+        }
+    }
+}
+
+// The tile's hidden layers (h1t, h2t) and outputs; samples past n count as zero
+// inputs.  h2 of this thread's 4 samples x 4 units stays in `h2`.
+__device__ __forceinline__ void forward_tile(TileShared& s, TileGrad* gr, const __half* x, uint32_t first,
+                                             uint32_t n, float (&h2)[4][4]) {
+    const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+    for (int i = threadIdx.x; i < kTile * F; i += kThreads) {
+        const uint32_t at = first + i / F;
+        const float v = at < n ? __half2float(x[(uint64_t)at * F + i % F]) : 0.f;
+        s.xt[i % F][i / F] = v;
+        if (gr) gr->x[i / F][i % F] = v;
+    }
+    __syncthreads();
+    float h1[4][4];
+    #pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        #pragma unroll
+        for (int b = 0; b < 4; ++b) h1[a][b] = s.b1[4 * tx + b];
+    }
+    product<F>(s.xt, s.w1t, ty, tx, h1);
+    #pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        #pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const float v = h1[a][b] > 0.f ? h1[a][b] : 0.f;
+            s.h1t[4 * tx + b][4 * ty + a] = v;
+            if (gr) gr->h1[4 * ty + a][4 * tx + b] = v;
+        }
+    }
+    __syncthreads();
+    #pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        #pragma unroll
+        for (int b = 0; b < 4; ++b) h2[a][b] = s.b2[4 * tx + b];
+    }
+    product<H>(s.h1t, s.w2t, ty, tx, h2);
+    #pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        #pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            h2[a][b] = h2[a][b] > 0.f ? h2[a][b] : 0.f;
+            s.h2t[4 * tx + b][4 * ty + a] = h2[a][b];
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < kTile) {
+        float o = s.b3;
+        #pragma unroll 8
+        for (int j = 0; j < H; ++j) o = fmaf(s.w3[j], s.h2t[j][threadIdx.x], o);
+        s.out[threadIdx.x] = o;
+    }
     __syncthreads();
 }
 
-// Forward pass, one thread per sample.  act (optional): h1, h2 per sample
-// (2H floats) for the backward pass.
-__global__ void __launch_bounds__(kBlock) forward_kernel(const __half* w, const __half* x,
-                                                         uint32_t n, float* act, float* out) {
-    __shared__ __half sw[NP];
-    stage_weights(w, sw);
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    float xin[F];
-    for (int f = 0; f < F; ++f) xin[f] = __half2float(x[(uint64_t)i * F + f]);
-    float h1[H];
-    for (int j = 0; j < H; ++j) {
-        float a = __half2float(sw[OFF_B1 + j]);
-        for (int f = 0; f < F; ++f) a = fmaf(__half2float(sw[OFF_W1 + j * F + f]), xin[f], a);
-        h1[j] = a > 0.f ? a : 0.f;
+// Forward pass.  What bounds it: latency (a few thousand samples are a few
+// tiles); one thread per sample ran its 5 000 multiply-adds one after the other.
+__global__ void __launch_bounds__(kThreads) forward_kernel(const __half* w, const __half* x, uint32_t n,
+                                                           float* out) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    TileShared& s = *reinterpret_cast<TileShared*>(smem);
+    load_weights(w, s);
+    const uint32_t tiles = (n + kTile - 1) / kTile;
+    for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+        const uint32_t first = t * kTile;
+        float h2[4][4];
+        forward_tile(s, nullptr, x, first, n, h2);
+        if (threadIdx.x < kTile && first + threadIdx.x < n) out[first + threadIdx.x] = s.out[threadIdx.x];
+        __syncthreads();
     }
-    float o = __half2float(sw[OFF_B3]);
-    for (int j = 0; j < H; ++j) {
-        float a = __half2float(sw[OFF_B2 + j]);
-        for (int q = 0; q < H; ++q) a = fmaf(__half2float(sw[OFF_W2 + j * H + q]), h1[q], a);
-        const float h2 = a > 0.f ? a : 0.f;
-        if (act) act[(uint64_t)i * 2 * H + H + j] = h2;
-        o = fmaf(__half2float(sw[OFF_W3 + j]), h2, o);
-    }
-    if (act)
-        for (int j = 0; j < H; ++j) act[(uint64_t)i * 2 * H + j] = h1[j];
-    out[i] = o;
 }
 
-// Backward pass of the mean squared error, one thread per sample; weight
-// gradients are summed per block in shared memory, then added to grad.
-__global__ void __launch_bounds__(kBlock) backward_kernel(const __half* w, const __half* x,
-                                                          const float* y, const float* act,
-                                                          const float* out, uint32_t n,
-                                                          float* grad, float* loss) {
-    __shared__ __half sw[NP];
-    __shared__ float sg[NP];
-    for (int p = threadIdx.x; p < NP; p += blockDim.x) sg[p] = 0.f;
-    stage_weights(w, sw);
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) {
-        const float* h1 = act + (uint64_t)i * 2 * H;
-        const float* h2 = h1 + H;
-        const float e = out[i] - y[i];
-        atomicAdd(loss, e * e / (float)n);
-        const float dout = 2.f * e / (float)n;
-        atomicAdd(&sg[OFF_B3], dout);
-        float dh2[H];
-        for (int j = 0; j < H; ++j) {
-            const float a = h2[j];
-            atomicAdd(&sg[OFF_W3 + j], dout * a);
-            dh2[j] = a > 0.f ? dout * __half2float(sw[OFF_W3 + j]) : 0.f;
-            if (dh2[j] != 0.f) atomicAdd(&sg[OFF_B2 + j], dh2[j]);
+// Forward and backward pass of the mean squared error over a block's tiles: the
+// block's sums of the weight gradients and of e^2, in FP32 registers until the
+// end, then NP + 1 values to part[block] (summed in a fixed order by
+// gradient_sum_kernel; the last one is the loss).
+//
+// What bounds it: FP32 multiply-adds (33 738 samples: 1.05 GFLOP, 15 us at the
+// chip's rate).  One thread per sample with one shared-memory atomic per sample
+// and weight took 2.1 ms of device time; this takes 0.04.
+__global__ void __launch_bounds__(kThreads) gradient_kernel(const __half* w, const __half* x, const float* y,
+                                                            uint32_t n, float* part) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    TileShared& s = *reinterpret_cast<TileShared*>(smem);
+    TileGrad& g = *reinterpret_cast<TileGrad*>(smem + (sizeof(TileShared) + 15) / 16 * 16);
+    const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
+    load_weights(w, s);
+    for (int i = tid; i < H * H; i += kThreads) g.w2[i / H][i % H] = __half2float(w[OFF_W2 + i]);
+    float dw2[4][4] = {}, dw1[4] = {}, dw3[4] = {}, db2[4] = {};   // dw2: [4 ty + a][4 tx + b] = [j][q]
+    float db1 = 0.f, db3 = 0.f, loss = 0.f;
+    const uint32_t tiles = (n + kTile - 1) / kTile;
+    for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
+        const uint32_t first = t * kTile;
+        float h2[4][4];
+        forward_tile(s, &g, x, first, n, h2);
+        if (tid < kTile) {
+            const float e = first + tid < n ? s.out[tid] - y[first + tid] : 0.f;
+            const float d = 2.f * e / (float)n;
+            g.dout[tid] = d;
+            loss += e * e / (float)n;
+            db3 += d;
         }
-        float xin[F];
-        for (int f = 0; f < F; ++f) xin[f] = __half2float(x[(uint64_t)i * F + f]);
-        for (int q = 0; q < H; ++q) {
-            const float a = h1[q];
-            float s = 0.f;
-            for (int j = 0; j < H; ++j) {
-                if (dh2[j] == 0.f) continue;
-                if (a != 0.f) atomicAdd(&sg[OFF_W2 + j * H + q], dh2[j] * a);
-                s = fmaf(__half2float(sw[OFF_W2 + j * H + q]), dh2[j], s);
+        __syncthreads();
+        // dh2 of this thread's 4 samples x 4 units
+        #pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            const float d = g.dout[4 * ty + a];
+            #pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                dw3[b] = fmaf(d, h2[a][b], dw3[b]);
+                const float v = h2[a][b] > 0.f ? d * s.w3[4 * tx + b] : 0.f;
+                db2[b] += v;
+                g.dh2[4 * ty + a][4 * tx + b] = v;
+                s.h2t[4 * tx + b][4 * ty + a] = v;
             }
-            const float dh1 = a > 0.f ? s : 0.f;
-            if (dh1 != 0.f) {
-                atomicAdd(&sg[OFF_B1 + q], dh1);
-                for (int f = 0; f < F; ++f) atomicAdd(&sg[OFF_W1 + q * F + f], dh1 * xin[f]);
+        }
+        __syncthreads();
+        product<kTile>(g.dh2, g.h1, ty, tx, dw2);
+        float dh1[4][4] = {};
+        product<H>(s.h2t, g.w2, ty, tx, dh1);
+        __syncthreads();   // every thread has read h1
+        #pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            #pragma unroll
+            for (int b = 0; b < 4; ++b)
+                g.h1[4 * ty + a][4 * tx + b] = s.h1t[4 * tx + b][4 * ty + a] > 0.f ? dh1[a][b] : 0.f;
+        }
+        __syncthreads();
+        // dw1[q][f .. f + 3]: q = tid / 4, f = 4 (tid % 4)
+        #pragma unroll 8
+        for (int i = 0; i < kTile; ++i) {
+            const float d = g.h1[i][tid >> 2];
+            const float4 v = *reinterpret_cast<const float4*>(&g.x[i][4 * (tid & 3)]);
+            dw1[0] = fmaf(d, v.x, dw1[0]); dw1[1] = fmaf(d, v.y, dw1[1]);
+            dw1[2] = fmaf(d, v.z, dw1[2]); dw1[3] = fmaf(d, v.w, dw1[3]);
+            if ((tid & 3) == 0) db1 += d;
+        }
+        __syncthreads();   // before the next tile's loads
+    }
+    float* p = part + (uint64_t)blockIdx.x * (NP + 1);
+    #pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        #pragma unroll
+        for (int b = 0; b < 4; ++b) p[OFF_W2 + (4 * ty + a) * H + 4 * tx + b] = dw2[a][b];
+        p[OFF_W1 + (tid >> 2) * F + 4 * (tid & 3) + a] = dw1[a];
+    }
+    if ((tid & 3) == 0) p[OFF_B1 + (tid >> 2)] = db1;
+    // sums over the 16 sample groups (ty), and over the samples
+    #pragma unroll 1
+    for (int b = 0; b < 4; ++b) {
+        #pragma unroll 1
+        for (int k = 0; k < 2; ++k) {
+            __syncthreads();
+            g.red[tx * 16 + ty] = k ? db2[b] : dw3[b];
+            __syncthreads();
+            if (ty == 0) {
+                float v = 0.f;
+                for (int i = 0; i < 16; ++i) v += g.red[tx * 16 + i];
+                p[(k ? OFF_B2 : OFF_W3) + 4 * tx + b] = v;
             }
         }
     }
-    __syncthreads();
-    for (int p = threadIdx.x; p < NP; p += blockDim.x)
-        if (sg[p] != 0.f) atomicAdd(&grad[p], sg[p]);
+    #pragma unroll 1
+    for (int k = 0; k < 2; ++k) {
+        __syncthreads();
+        g.red[tid] = k ? loss : db3;
+        __syncthreads();
+        if (tid == 0) {
+            float v = 0.f;
+            for (int i = 0; i < kTile; ++i) v += g.red[i];
+            p[k ? NP : OFF_B3] = v;
+        }
+    }
+}
+
+// grad[p] = sum over blocks of part[.][p]; loss = the last column.  One warp per
+// 8 parameters, 4 lanes each, so that the loads of a column overlap.
+__global__ void gradient_sum_kernel(const float* part, uint32_t blocks, float* grad, float* loss) {
+    const uint32_t p = (blockIdx.x * blockDim.x + threadIdx.x) >> 2, lane = threadIdx.x & 3u;
+    float v = 0.f;
+    if (p <= NP) {
+        #pragma unroll 4
+        for (uint32_t i = lane; i < blocks; i += 4) v += part[(uint64_t)i * (NP + 1) + p];
+    }
+    v += __shfl_xor_sync(0xFFFFFFFFu, v, 1);
+    v += __shfl_xor_sync(0xFFFFFFFFu, v, 2);
+    if (lane == 0 && p <= NP) *(p < NP ? grad + p : loss) = v;
 }
 
 // Adam step on the FP32 master weights; refreshes the FP16 copy.
