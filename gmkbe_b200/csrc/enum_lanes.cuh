@@ -14,8 +14,10 @@
 //     That row is filtered once per call into a list (ws) of ids and masks of
 //     missed members: entries above c are candidates, the others outsiders;
 //   * vertices of side o come from the row of a saturated member of S_s
-//     (filtered once into the list wo) or, when c itself has k misses, from
-//     c's own row, walked by its lane;
+//     (filtered once into the list wo, with the misses between the two lists,
+//     and their rows walked along as the members' are: no probe is left in the
+//     block) or, when c itself has k misses, from c's own row, walked by its
+//     lane;
 //   * with m <= kLaneC candidates, every subset T is tested.  All lanes are at
 //     the same T.  A vertex is a bit: members 0..ns-1, c at ns, candidates
 //     from 16; miss counts of all vertices are kept bit-sliced in four words,
@@ -51,7 +53,9 @@ struct LaneShared {
     uint32_t ids[16], off[16], deg[16];     // the members, their rows
     uint32_t cursor[16];                    // S_o's rows: the first entry >= the next block's base
     uint32_t ws_id[kLaneList], ws_m[kLaneList];
-    uint32_t wo_id[kLaneList], wo_m[kLaneList];
+    uint32_t wo_id[kLaneRow], wo_m[kLaneRow];
+    uint32_t wo_at[kLaneRow], wo_end[kLaneRow];   // wo's rows, as cursors into adj
+    uint32_t ws_miss[kLaneList];            // wo entries that each ws entry misses
     uint32_t own, opp, sat0, ss;            // members on c's side, on the other; one miss left; at k
     uint32_t z0, zs;                        // lowest-degree members of sat0 and ss (zs 32: none)
     uint32_t nws, nwo, listed;
@@ -62,6 +66,7 @@ struct LaneShared {
 // ... and what only deciding a block needs (the bit search's words).
 struct LaneScratch {
     uint32_t cid[kLaneC][32], cw[kLaneC][32];
+    uint32_t cq[kLaneC][32];                // ws position of the candidates of c's side
     uint32_t ow[kLaneO][32];
 };
 
@@ -229,6 +234,29 @@ __device__ __forceinline__ void lane_blocks(Ctx& t, const Outputs& o, uint32_t c
                 sh.miss[0] = p0; sh.miss[1] = p1; sh.miss[2] = p2; sh.miss[3] = p3;
                 sh.a = a_s; sh.b = b_s;
             }
+            if (listed) {
+                // wo's rows from pos on (lane q searches row q), and the misses
+                // between ws and wo, one ws entry per lane
+                const uint32_t nwo = sh.nwo, nws = sh.nws;
+                if (lane < nwo) {
+                    const uint32_t w = sh.wo_id[lane], end_w = g.off[w + 1];
+                    uint32_t lo = g.off[w], hi = end_w;
+                    while (lo < hi) {
+                        const uint32_t mid_w = lo + ((hi - lo) >> 1);
+                        if (g.adj[mid_w] < pos) lo = mid_w + 1; else hi = mid_w;
+                    }
+                    sh.wo_at[lane] = lo;
+                    sh.wo_end[lane] = end_w;
+                }
+                #pragma unroll 1
+                for (uint32_t q = lane; q < nws; q += 32) {
+                    const uint32_t v = sh.ws_id[q];
+                    uint32_t m = 0;
+                    #pragma unroll 1
+                    for (uint32_t i = 0; i < nwo; ++i) m |= adj_test(t, v, sh.wo_id[i]) ? 0u : 1u << i;
+                    sh.ws_miss[q] = m;
+                }
+            }
             // the first entries of S_o's rows that are >= pos
             #pragma unroll 1
             for (uint32_t y = opp; y; y &= y - 1) {
@@ -284,7 +312,7 @@ __device__ __forceinline__ void lane_blocks(Ctx& t, const Outputs& o, uint32_t c
         for (uint32_t q = 0; q < nws; ++q) {
             const uint32_t v = sh.ws_id[q], mv = sh.ws_m[q];
             if (local && v > c && !(mv & satc)) {
-                if (m < kLaneC) { sc.cid[m][lane] = v; sc.cw[m][lane] = mv; }
+                if (m < kLaneC) { sc.cid[m][lane] = v; sc.cw[m][lane] = mv; sc.cq[m][lane] = q; }
                 ++m;
             }
         }
@@ -299,18 +327,19 @@ __device__ __forceinline__ void lane_blocks(Ctx& t, const Outputs& o, uint32_t c
         if (listed) {
             #pragma unroll 1
             for (uint32_t q = 0; q < nwo; ++q) {
-                const uint32_t w = sh.wo_id[q];
+                const uint32_t at = sh.wo_at[q], p = at + lane;
+                const uint32_t e = p < sh.wo_end[q] ? g.adj[p] - pbase : kFull;
+                const uint32_t adj = __reduce_or_sync(kFull, e < 32 ? 1u << e : 0u);
+                if (lane == 0) sh.wo_at[q] = at + __popc(adj);
                 uint32_t mw = sh.wo_m[q];
-                if (simple) {
-                    const bool a = adj_test(t, w, c);
-                    if (!a) mw |= 1u << ns;
-                    if ((uint32_t)__popc(mw) <= k && (a || mcc < k)) {
-                        #pragma unroll 1
-                        for (uint32_t j = 0; j < mcs; ++j)
-                            if (!adj_test(t, w, sc.cid[j][lane])) mw |= 1u << (16 + j);
-                        if (no < kLaneO) sc.ow[no][lane] = mw;
-                        ++no;
-                    }
+                const bool a = (adj >> lane) & 1u;
+                if (!a) mw |= 1u << ns;
+                if (simple && (uint32_t)__popc(mw) <= k && (a || mcc < k)) {
+                    #pragma unroll 1
+                    for (uint32_t j = 0; j < mcs; ++j)
+                        mw |= ((sh.ws_miss[sc.cq[j][lane]] >> q) & 1u) << (16 + j);
+                    if (no < kLaneO) sc.ow[no][lane] = mw;
+                    ++no;
                 }
             }
         } else {
