@@ -295,6 +295,20 @@ __device__ __forceinline__ void arena_full(Ctx& t, uint32_t cur, uint32_t site, 
     t.err = TASK_ARENA_FULL;
 }
 
+// In a loop over a long list or row (`base` its 32-entry position): has the run
+// (or this graph) been stopped?  A hub's row of tens of thousands of entries,
+// each with its probes, takes milliseconds, and a run that has its results must
+// not wait for it.  Looked at every 1 024 entries; the task is then dropped.
+constexpr int TASK_STOPPED = 98;
+__device__ __forceinline__ bool stopped(Ctx& t, const Outputs& o, uint32_t base) {
+    if ((base & 1023u) != 992u) return false;
+    int stop = 0;
+    if (t.lane == 0) stop = load_flag(o.stop) || (o.gstop && load_flag(o.gstop));
+    if (!bcast(stop)) return false;
+    t.err = TASK_STOPPED;
+    return true;
+}
+
 __device__ void fail(Ctx& t, const Outputs& o, int code) {
     if (!t.err) t.err = code;
     if (t.lane == 0) {
@@ -574,8 +588,8 @@ __device__ bool outsider_addable(Ctx& t, const uint32_t* l0, uint32_t n0, const 
 // Warp form of outsider_addable_mixed (enum_core.cuh): side s global (ids >
 // lo), side o local (list l, n entries).  Scratch at `tot`: n list totals,
 // then the S_o member ids and their totals (2 ns words).
-__device__ bool outsider_addable_mixed(Ctx& t, int s, uint32_t lo, const uint32_t* l, uint32_t n,
-                                       uint32_t* tot) {
+__device__ bool outsider_addable_mixed(Ctx& t, const Outputs& out, int s, uint32_t lo, const uint32_t* l,
+                                       uint32_t n, uint32_t* tot) {
     const GraphView& g = t.g;
     const int o = 1 - s;
     const uint32_t G = side_end(g, s) - lo - 1;
@@ -603,6 +617,7 @@ __device__ bool outsider_addable_mixed(Ctx& t, int s, uint32_t lo, const uint32_
     }
     #pragma unroll 1
     for (uint32_t base = 0; base < n; base += 32) {
+        if (stopped(t, out, base)) return true;
         const uint32_t q = base + t.lane;
         if (q < n) {
             const uint32_t w = l[2 * q];
@@ -638,6 +653,7 @@ __device__ bool outsider_addable_mixed(Ctx& t, int s, uint32_t lo, const uint32_
         if (t.lane == 0) t.work += d;
         #pragma unroll 1
         for (uint32_t base = 0; base < d; base += 32) {
+            if (stopped(t, out, base)) return true;
             const uint32_t p = base + t.lane;
             bool ok = false, past = false;
             if (p < d) {
@@ -831,19 +847,19 @@ __device__ __forceinline__ uint32_t bits_region(const Ctx& t, uint32_t cur, cons
 }
 
 // Builds the bitmaps of frame cur (called when it starts branching).
-__device__ __forceinline__ void add_filter_bits(Ctx& t, uint32_t cur, const Hdr& f) {
+__device__ __forceinline__ void add_filter_bits(Ctx& t, const Outputs& o, uint32_t cur, const Hdr& f) {
     uint32_t top = f.top, flags = 0;
     #pragma unroll 1
     for (int s = 0; s < 2; ++s) {
         const uint32_t n = f.cnt.get(s);
         if ((f.flags & gbit(s)) || n < t.bits_min) continue;
-        const int o = 1 - s;
-        // Z: members of side o at k - 1 misses, in S order
+        const int os = 1 - s;
+        // Z: members of side os at k - 1 misses, in S order
         uint32_t nz = 0;
         #pragma unroll 1
         for (uint32_t base = 0; base < t.ns; base += 32) {
             const uint32_t i = base + t.lane;
-            const bool on = i < t.ns && side_of(t.g, t.sid[i]) == o && t.smc[i] + 1 == t.k;
+            const bool on = i < t.ns && side_of(t.g, t.sid[i]) == os && t.smc[i] + 1 == t.k;
             const uint32_t mask = __ballot_sync(kFull, on);
             if (on) {
                 const uint32_t r = nz + __popc(mask & lanemask_lt());
@@ -864,6 +880,7 @@ __device__ __forceinline__ void add_filter_bits(Ctx& t, uint32_t cur, const Hdr&
             uint32_t end = 0;
             #pragma unroll 1
             for (uint32_t base = 0; base < n; base += 32) {
+                if (stopped(t, o, base)) return;
                 const uint32_t q = base + t.lane;
                 const bool a = q < n && adj_test(t, lst[2 * q], z);
                 const uint32_t word = __ballot_sync(kFull, a);
@@ -920,6 +937,7 @@ __device__ uint32_t build_child(Ctx& t, const Outputs& o, uint32_t cur, uint32_t
             const uint32_t* row = g.adj + g.off[z];
             #pragma unroll 1
             for (uint32_t base = 0; base < dz; base += 32) {
+                if (stopped(t, o, base)) return kNoPos;
                 const uint32_t q = base + t.lane;
                 bool keep = false;
                 uint32_t v = 0, m = 0;
@@ -1003,6 +1021,7 @@ __device__ uint32_t build_child(Ctx& t, const Outputs& o, uint32_t cur, uint32_t
         } else {
             #pragma unroll 1
             for (uint32_t base = start; base < n; base += 32) {
+                if (stopped(t, o, base - start)) return kNoPos;
                 const uint32_t q = base + t.lane;
                 bool keep = false;
                 uint32_t v = 0, m = 0;
@@ -1052,6 +1071,7 @@ __device__ uint32_t build_child(Ctx& t, const Outputs& o, uint32_t cur, uint32_t
                 if (t.lane == 0) t.work += d;
                 #pragma unroll 1
                 for (uint32_t base = 0; base < d; base += 32) {
+                    if (stopped(t, o, base)) return kNoPos;
                     const uint32_t e = base + t.lane;
                     bool keep = false;
                     uint32_t v = 0, mm = 0;
@@ -1077,6 +1097,7 @@ __device__ uint32_t build_child(Ctx& t, const Outputs& o, uint32_t cur, uint32_t
         if (w + 2ull * n > t.cap) { arena_full(t, cur, kSiteChild, c); return kNoPos; }
         #pragma unroll 1
         for (uint32_t base = 0; base < n; base += 32) {
+            if (stopped(t, o, base)) return kNoPos;
             const uint32_t q = base + t.lane;
             bool keep = false;
             uint32_t v = 0, m = 0;
@@ -1198,7 +1219,7 @@ __device__ int enter_node(Ctx& t, const Outputs& o, uint32_t cur, ChildReq* req,
         const uint32_t n = f.cnt.get(os);
         const uint32_t base = f.top;
         if (base + n + 2ull * t.ns > t.cap) { arena_full(t, cur, kSiteNode, 0); return ENTER_DONE; }
-        if (outsider_addable_mixed(t, s, f.lo.get(s), t.arena + f.off.get(os), n, t.arena + base))
+        if (outsider_addable_mixed(t, o, s, f.lo.get(s), t.arena + f.off.get(os), n, t.arena + base))
             return ENTER_DONE;
     }
     if (!g0 && !g1) {
@@ -1337,7 +1358,7 @@ __device__ int enter_node(Ctx& t, const Outputs& o, uint32_t cur, ChildReq* req,
     }
     __syncwarp();
     if (kBits && ((!g0 && f.cnt.a >= t.bits_min) || (!g1 && f.cnt.b >= t.bits_min)))
-        add_filter_bits(t, cur, f);
+        add_filter_bits(t, o, cur, f);
     return ENTER_ITERATE;
 }
 

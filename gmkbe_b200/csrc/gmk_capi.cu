@@ -439,6 +439,7 @@ enumerate_warp_kernel(const __grid_constant__ WarpArgs a) {
         // five atomics on one line per task would cost short tasks more than
         // their search
         if (kBatch || o.limit) flush(t, o);
+        if (t.err == TASK_STOPPED) t.err = 0;   // (a batch goes on with its other graphs)
         if (t.err) break;
     }
     flush(t, o);

@@ -85,3 +85,20 @@ def test_larger_than_the_small_graph_search():
             assert dg.enumerate(k=1, schedule="ordered", task_cost=cost).summary() == want
             got = G.enumerate_batch([dg], [1])[0]
             assert got.summary() == want
+
+
+def test_a_reached_limit_ends_long_rows():
+    # three V hubs adjacent to 20 000 U vertices: lists of that length are being
+    # built when the limit is reached, and those tasks are dropped; the run, and
+    # in a batch the graph, stops at its cap while the other graph runs to its end
+    hub = gg.hubs_and_sparse(3, 40, 20_000, 3, 6)
+    small = gg.erdos_renyi(12, 140, 2.0 / 140, 9)
+    want = O.enumerate_oracle(small, 1).summary()
+    with G.Graph.from_graph(hub) as h, G.Graph.from_graph(small) as s:
+        for limit in (1, 1000, 200_000):
+            st = h.enumerate(k=2, result_limit=limit)
+            assert st.count == limit and st.truncated
+        got = G.enumerate_batch([h, s], [2, 1], limits=[5000, 0])
+        assert got[0].count == 5000 and got[0].truncated
+        assert got[1].summary() == want and not got[1].truncated
+        assert h.enumerate(k=2, result_limit=50, collect=True).count == 50
