@@ -16,27 +16,31 @@
 //   forced                   candidates with at most k misses that miss no
 //                            vertex with more than k are in every maximal leaf
 //   at most 5 candidates     every subset of them is tested, one per lane
-//   branch                   take the included vertex with the most misses
+//   branch                   take the included vertex v with the most misses
 //                            (over k; at most k of them can stay), and of the
 //                            candidates it misses the one with the most misses:
 //                            it is included, or it is excluded
+//   fan                      when v has one miss left, at most one of the
+//                            candidates P it misses can be included: one child
+//                            per w in P (the rest of P is out, v has k misses
+//                            then) and the state without P
 // Root task: x in U with I = {x}, C = the U vertices after x and all V
 // vertices, or, for a range of first-level children y, one state (x, y) after
 // the other (C: after x, after y).
 //
 // States waiting on the warp's stack are handed to idle warps (tickets and
-// slots, as in the list-based kernel; a record is one state, and its slot
+// slots, as in the list-based kernel; a record is one stack entry, and its slot
 // holds it, so there is no separate index).
 //
 // What bounds it: integer issue, and on graphs of a few thousand nodes the
 // latency of one warp's chain of nodes.  The list-based search of the same
 // graphs spent 1 000-1 600 warp instructions a node on hash probes, frames and
-// lists, and their L2 latency; this one spends 640 with N = 3 masks (77 x 77, k
-// = 2: 10.3 G instructions for 12.4 M results, 43 % of the issue slots active)
-// and nothing leaves the SM.  Measured, complete runs, list-based -> here (ms,
-// one B200): 18 x 14 k = 1 0.90 -> 0.14, k = 3 19.5 -> 0.29; 58 x 58 k = 2 30.3 ->
-// 2.9; 77 x 77 k = 2 115 -> 14.2; 82 x 83 k = 2 31.6 -> 13.9; 128 x 128 k = 1
-// 10.4 -> 2.8.
+// lists, and their L2 latency; this one spent 640 with N = 3 masks (77 x 77, k
+// = 2, before the fans: 10.3 G instructions for 12.4 M results, 43 % of the
+// issue slots active) and nothing leaves the SM.  Measured, complete runs, list-based -> here (ms,
+// one B200): 18 x 14 k = 1 0.90 -> 0.13, k = 3 19.5 -> 0.29; 58 x 58 k = 2 30.3 ->
+// 2.35; 77 x 77 k = 2 115 -> 10.6; 82 x 83 k = 2 31.6 -> 8.5; 128 x 128 k = 1
+// 10.4 -> 2.2.
 #pragma once
 #include "enum_warp.cuh"
 
@@ -59,11 +63,28 @@ constexpr uint32_t kShareMax = 8;      // states handed on per look, at most
 // N use one record size: a record is recognised by the launch number in its
 // first word, which must never have been another launch's state word.
 constexpr uint32_t kHeader = 4;
-constexpr uint32_t kRecordWords = kHeader + 16;
+constexpr uint32_t kRecordWords = kHeader + 21;
 // Stack entries in shared memory; deeper ones are in the warp's global spill
-// area.  One entry per included candidate on the path.
+// area.  One entry per included candidate on the path (a fan leaves one for all
+// its children, and each has fewer candidates).
 template <int N> __host__ __device__ constexpr uint32_t shared_depth() { return N == 1 ? 64 : N == 2 ? 32 : 16; }
-template <int N> __host__ __device__ constexpr uint32_t spill_words() { return (64 * N - shared_depth<N>()) * 4 * N; }
+// Fans (the children that include one of P each, and the state without P, in
+// place of a chain of include / exclude states) where P has 6 vertices or more:
+// the chain's exclude states are nodes that decide nothing, -41 % nodes at 60 x
+// 60, 180 edges, k = 2: 2.98 to 2.35 ms; 80 x 80, 320 edges, k = 2: 14.3 to
+// 10.6; 50 x 50, 120 edges, k = 3: 174 to 125; 128 x 128, 1200 edges, k = 1: 2.79
+// to 2.19.  From 4 on: 2.06 at the last, but 0.51 in place of 0.47 ms at 60 x
+// 60, 300 edges, k = 1; from 8 on: 2.4 and 0.47.  With one word a side the run is
+// a chain of few states and a fan is handed on as a whole: 30 x 30, 155 edges, k =
+// 1 takes 0.23 ms with fans and 0.17 without.
+template <int N> constexpr bool kFans = N > 1;
+constexpr uint32_t kFanMin = 6;
+// An entry: a state, and the children of a fan that are still to be searched
+// before it (their mask, and its side: 0 none, 1 U, 2 V).
+template <int N> __host__ __device__ constexpr uint32_t entry_words() { return kFans<N> ? 5 * N + 1 : 4 * N; }
+template <int N> __host__ __device__ constexpr uint32_t spill_words() {
+    return (64 * N - shared_depth<N>()) * entry_words<N>();
+}
 
 template <int N>
 struct State {
@@ -72,7 +93,7 @@ struct State {
 
 template <int N>
 struct Shared {
-    uint32_t stack[shared_depth<N>()][4 * N];
+    uint32_t stack[shared_depth<N>()][entry_words<N>()];
     uint32_t found[64][2 * N];                     // results not yet hashed: U and V masks
     unsigned long long ea[64 * N], eb[64 * N];     // hash elements (U at 0, V at 32 N)
 };
@@ -308,16 +329,18 @@ __device__ __forceinline__ bool subsets(const Ctx<N>& t, const State<N>& s, uint
 
 template <int N>
 __device__ __forceinline__ uint32_t* stack_at(const Ctx<N>& t, uint32_t i) {
-    return i < shared_depth<N>() ? t.sh->stack[i] : t.spill + (i - shared_depth<N>()) * 4 * N;
+    return i < shared_depth<N>() ? t.sh->stack[i] : t.spill + (i - shared_depth<N>()) * entry_words<N>();
 }
 template <int N>
-__device__ __forceinline__ void push(Ctx<N>& t, const State<N>& s) {
+__device__ __forceinline__ void push(Ctx<N>& t, const State<N>& s, const uint32_t (&p)[N], uint32_t side) {
     uint32_t* e = stack_at<N>(t, t.sp);
     if (t.lane == 0) {
         #pragma unroll
         for (int w = 0; w < N; ++w) {
             e[w] = s.iu[w]; e[N + w] = s.iv[w]; e[2 * N + w] = s.cu[w]; e[3 * N + w] = s.cv[w];
+            if (kFans<N> && side) e[4 * N + w] = p[w];
         }
+        if (kFans<N>) e[5 * N] = side;
     }
     ++t.sp;
 }
@@ -329,10 +352,53 @@ __device__ __forceinline__ void read_state(const uint32_t* e, State<N>& s) {
     }
 }
 
-// One node: prunes, takes results, or goes down to the child that includes the
-// branching candidate (true; the state that excludes it is pushed).
+// The next waiting state: the top entry's first remaining child (true: to be
+// refitted), else its state.
 template <int N>
-__device__ __forceinline__ bool node(Ctx<N>& t, State<N>& s) {
+__device__ __forceinline__ bool pop(Ctx<N>& t, State<N>& s) {
+    if (!kFans<N>) {
+        --t.sp;
+        __syncwarp();
+        read_state<N>(stack_at<N>(t, t.sp), s);
+        __syncwarp();
+        return false;
+    }
+    __syncwarp();
+    uint32_t* e = stack_at<N>(t, t.sp - 1);
+    read_state<N>(e, s);
+    const uint32_t side = e[5 * N];
+    if (side == 0) {
+        --t.sp;
+        __syncwarp();
+        return false;
+    }
+    uint32_t bit = 0, left = 0;
+    int word = 0;
+    #pragma unroll
+    for (int w = N - 1; w >= 0; --w) {
+        const uint32_t p = e[4 * N + w];
+        left = p ? left | bit | (p & (p - 1)) : left;
+        if (p) { word = w; bit = p & (0u - p); }
+    }
+    #pragma unroll
+    for (int w = 0; w < N; ++w) {
+        const uint32_t m = word == w ? bit : 0u;
+        if (side == 1) s.iu[w] |= m; else s.iv[w] |= m;
+    }
+    __syncwarp();
+    if (t.lane == 0) {
+        e[4 * N + word] &= ~bit;
+        if (!left) e[5 * N] = 0;
+    }
+    return true;
+}
+
+// One node: prunes, takes results, or goes on to another state (true): the child
+// that includes the branching candidate (the state that excludes it is pushed),
+// or, after a fan whose children are all done, the state without them.
+template <int N>
+__device__ __forceinline__ bool node(Ctx<N>& t, State<N>& s, bool fit) {
+    if (kFans<N> && fit) refit<N>(t, s);
     const uint32_t lane = t.lane, k = t.k;
     uint32_t lu[N], lv[N], tu[N], tv[N], hu[N], hv[N], bu[N], bv[N];
     uint32_t any_v = 0, any_b = 0;
@@ -385,6 +451,8 @@ __device__ __forceinline__ bool node(Ctx<N>& t, State<N>& s) {
             for (int w = 0; w < N; ++w) { pu[w] = s.cu[w]; pv[w] = s.cv[w]; }
             if (best) {
                 const uint32_t at = 255u - (best & 255u);   // U at 0, V at 128
+                const bool on_u = at < 128;
+                uint32_t cur = 0, np = 0;
                 #pragma unroll
                 for (int w = 0; w < N; ++w) {
                     uint32_t mu = 0, mv = 0;
@@ -392,10 +460,23 @@ __device__ __forceinline__ bool node(Ctx<N>& t, State<N>& s) {
                     for (int i = 0; i < N; ++i) {
                         if (((at & 127u) >> 5) == (uint32_t)i) { mu = t.um[i][w]; mv = t.vm[i][w]; }
                     }
-                    mu = __shfl_sync(kFull, mu, at & 31u);
-                    mv = __shfl_sync(kFull, mv, at & 31u);
-                    pu[w] &= at < 128 ? 0u : mv;
-                    pv[w] &= at < 128 ? mu : 0u;
+                    const uint32_t m = __shfl_sync(kFull, on_u ? mu : mv, at & 31u);
+                    pu[w] &= on_u ? 0u : m;
+                    pv[w] &= on_u ? m : 0u;
+                    cur += __popc(m & (on_u ? s.iv[w] : s.iu[w]));
+                    np += __popc(pu[w] | pv[w]);
+                }
+                if (kFans<N> && cur + 1 == k && np >= kFanMin) {
+                    // a fan: at most one of p
+                    uint32_t p[N];
+                    #pragma unroll
+                    for (int w = 0; w < N; ++w) {
+                        p[w] = on_u ? pv[w] : pu[w];
+                        s.cu[w] &= ~pu[w];
+                        s.cv[w] &= ~pv[w];
+                    }
+                    push<N>(t, s, p, on_u ? 2u : 1u);
+                    return false;
                 }
             }
             best = 0;
@@ -413,13 +494,13 @@ __device__ __forceinline__ bool node(Ctx<N>& t, State<N>& s) {
                 const uint32_t m = word == (uint32_t)w ? bit : 0u;
                 if (at < 128) s.cu[w] &= ~m; else s.cv[w] &= ~m;
             }
-            push<N>(t, s);
+            push<N>(t, s, pu, 0u);
             #pragma unroll
             for (int w = 0; w < N; ++w) {
                 const uint32_t m = word == (uint32_t)w ? bit : 0u;
                 if (at < 128) s.iu[w] |= m; else s.iv[w] |= m;
             }
-            refit<N>(t, s);
+            if (!kFans<N>) refit<N>(t, s);
             return true;
         }
         uint32_t feasible;
@@ -437,8 +518,8 @@ __device__ __forceinline__ bool node(Ctx<N>& t, State<N>& s) {
     return false;
 }
 
-// Hands up to `want` of the oldest waiting states (those with kMinShare
-// candidates or more) to waiting warps.
+// Hands up to `want` of the oldest entries (those with kMinShare candidates
+// and children or more) to waiting warps.
 template <int N>
 __device__ __forceinline__ void donate(Ctx<N>& t, const Share& sh, uint32_t gid, uint32_t want) {
     __syncwarp();
@@ -451,6 +532,10 @@ __device__ __forceinline__ void donate(Ctx<N>& t, const Share& sh, uint32_t gid,
         const uint32_t* e = stack_at<N>(t, t.bottom + t.lane);
         #pragma unroll
         for (int w = 2 * N; w < 4 * N; ++w) c += __popc(e[w]);
+        if (kFans<N> && e[5 * N]) {
+            #pragma unroll
+            for (int w = 4 * N; w < 5 * N; ++w) c += __popc(e[w]);
+        }
     }
     const uint32_t small = __ballot_sync(kFull, t.lane >= n || c < kMinShare);
     n = __ffs(small) - 1;      // (n <= kShareMax < 32: some lane is set)
@@ -474,7 +559,7 @@ __device__ __forceinline__ void donate(Ctx<N>& t, const Share& sh, uint32_t gid,
         const uint32_t* e = stack_at<N>(t, t.bottom + t.lane);
         r[1] = gid;
         #pragma unroll
-        for (int w = 0; w < 4 * N; ++w) r[kHeader + w] = e[w];
+        for (uint32_t w = 0; w < entry_words<N>(); ++w) r[kHeader + w] = e[w];
         __threadfence();
         atomicExch(r, sh.launch);
     }

@@ -524,8 +524,8 @@ enumerate_dense_kernel(const __grid_constant__ DenseArgs a) {
         j = bcast(j);
         if (stop) break;
         State<N> s;
-        uint32_t next_gid = 0, root = 0, y = 0, y_end = 0;
-        bool have = true;
+        uint32_t next_gid = 0, root = 0, y = 0, y_end = 0, sp = 0;
+        bool have = true, fit = true;
         if (j >= a.queue_len) {
             // take a ticket and wait for its slot's record, or for the end of
             // the launch's work (no task outstanding)
@@ -575,6 +575,12 @@ enumerate_dense_kernel(const __grid_constant__ DenseArgs a) {
                 s.iu[w] = __ldcg(r + kHeader + w); s.iv[w] = __ldcg(r + kHeader + N + w);
                 s.cu[w] = __ldcg(r + kHeader + 2 * N + w); s.cv[w] = __ldcg(r + kHeader + 3 * N + w);
             }
+            if (kFans<N>) {
+                // (with its children: the bottom of this warp's stack)
+                if (lane < entry_words<N>()) stack_at<N>(t, 0)[lane] = __ldcg(r + kHeader + lane);
+                have = false;
+                sp = 1;
+            }
         } else {
             if (lane == 0) atomicAdd(&a.rc->tasks_done, 1ull);
             TaskEntry e{0, 0, 0, 0};
@@ -622,12 +628,17 @@ enumerate_dense_kernel(const __grid_constant__ DenseArgs a) {
         #pragma unroll
         for (int w = N - 1; w >= 0; --w)
             if (s.iu[w]) root = 32 * w + __ffs(s.iu[w]) - 1;
-        t.sp = t.bottom = t.extra = 0;
+        t.sp = kFans<N> ? sp : 0;
+        t.bottom = t.extra = 0;
         uint32_t polls = 0;
         unsigned long long nodes = 0;
         bool quit = kBatch && gmk::load_flag(&ctr->stop);   // a capped graph's tasks end at once
         quit = __any_sync(gmk::warp::kFull, quit);
         while (!quit) {
+            if (kFans<N> && !have && t.sp != t.bottom) {
+                fit = pop<N>(t, s);
+                have = true;
+            }
             if (!have) {
                 if (y >= y_end) break;
                 // the next first-level child: after x, after y
@@ -639,9 +650,9 @@ enumerate_dense_kernel(const __grid_constant__ DenseArgs a) {
                     s.cu[w] = low_bits(nl, w) & ~low_bits(root + 1, w);
                     s.cv[w] = low_bits(nv, w) & ~low_bits(y + 1, w);
                 }
-                refit<N>(t, s);
+                if (!kFans<N>) refit<N>(t, s);
                 ++y;
-                have = true;
+                have = fit = true;
             }
             if (++polls == poll_nodes<N>()) {
                 polls = 0;
@@ -665,19 +676,10 @@ enumerate_dense_kernel(const __grid_constant__ DenseArgs a) {
                 if (limit && t.cnt >= gmk::kFlushBatch) flush();
             }
             ++nodes;
-            const bool down = node<N>(t, s);
+            have = fit = node<N>(t, s, fit);
             nodes += t.extra;
             t.extra = 0;
-            if (!down) {
-                if (t.sp == t.bottom) {
-                    have = false;
-                } else {
-                    --t.sp;
-                    __syncwarp();
-                    read_state<N>(stack_at<N>(t, t.sp), s);
-                    __syncwarp();
-                }
-            }
+            if (!kFans<N> && !have && t.sp != t.bottom) have = !pop<N>(t, s);
         }
         t.nodes += nodes;
         if (lane == 0) {

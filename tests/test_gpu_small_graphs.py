@@ -122,3 +122,21 @@ def test_batches_of_small_graphs_and_mixed_sizes():
     finally:
         for dg in dgs:
             dg.close()
+
+
+@pytest.mark.parametrize("nu,nv,m,k", [(32, 33, 60, 2), (33, 32, 150, 1), (64, 65, 200, 1), (40, 33, 70, 2),
+                                       (34, 12, 60, 3), (96, 97, 330, 1), (128, 127, 400, 1), (65, 20, 90, 2)])
+def test_fans_of_children(nu, nv, m, k):
+    # sparse sides over a mask word: an included vertex misses many candidates,
+    # of which one at most can join; whole, shared early, in parts and cut off
+    rng = np.random.default_rng(nu * nv + k)
+    u = np.concatenate([np.arange(nu), rng.integers(0, nu, m - nu)])
+    v = np.concatenate([np.arange(nu) % nv, rng.integers(0, nv, m - nu)])
+    g = gg.relabel(u, v)
+    with G.Graph.from_graph(g) as dg:
+        want = dg.enumerate(k=k, sharing=False).summary()
+        for kw in (dict(), dict(donate_min_nodes=64), dict(chunk=3), dict(threads=32), dict(schedule="plain")):
+            assert dg.enumerate(k=k, **kw).summary() == want, kw
+        st = dg.enumerate(k=k, result_limit=want[0] // 2)
+        assert st.count == want[0] // 2 and st.truncated
+        assert [s.summary() for s in G.enumerate_batch([dg, dg], [k, k])] == [want, want]
