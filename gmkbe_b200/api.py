@@ -76,6 +76,11 @@ class _Task(ctypes.Structure):
                 ("graph", ctypes.c_uint32), ("cost", ctypes.c_float)]
 
 
+class _Collector(ctypes.Structure):
+    _fields_ = [("data", ctypes.c_void_p), ("len", ctypes.c_uint64), ("cap", ctypes.c_uint64),
+                ("failed", ctypes.c_int32)]
+
+
 SINK = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_void_p, ctypes.POINTER(ctypes.c_uint32),
                         ctypes.c_uint32, ctypes.POINTER(ctypes.c_uint32), ctypes.c_uint32)
 
@@ -98,6 +103,8 @@ def load_library(path: str = LIB_PATH):
     lib.gmk_graph_fingerprint.argtypes = [ctypes.c_void_p, ctypes.POINTER(ctypes.c_uint64)]
     lib.gmk_graph_free.argtypes = [ctypes.c_void_p]
     lib.gmk_graph_free.restype = None
+    lib.gmk_collect_free.argtypes = [ctypes.c_void_p]
+    lib.gmk_collect_free.restype = None
     lib.gmk_opts_default.argtypes = [ctypes.POINTER(_Opts)]
     lib.gmk_opts_default.restype = None
     lib.gmk_enumerate.argtypes = [ctypes.c_void_p, ctypes.POINTER(_Opts), SINK, ctypes.c_void_p,
@@ -323,18 +330,42 @@ class Graph:
         return o, cost
 
     @staticmethod
-    def _sink(collect, sink, out):
-        if not (collect or sink is not None):
-            return SINK(0)
+    def _sink(collect, sink, store):
+        """The record callback and its user pointer: the library's own collector
+        (into store), the caller's sink, or none."""
+        if collect:
+            return SINK(("gmk_collect", load_library())), ctypes.addressof(store)
+        if sink is None:
+            return SINK(0), None
 
         def _cb(_u, xp, nx, yp, ny):
-            x = tuple(xp[i] for i in range(nx))
-            y = tuple(yp[i] for i in range(ny))
-            if collect:
-                out.append((x, y))
-                return 0
-            return 1 if sink(x, y) else 0
-        return SINK(_cb)
+            return 1 if sink(tuple(xp[:nx]), tuple(yp[:ny])) else 0
+        return SINK(_cb), None
+
+    @staticmethod
+    def _records(store, slab=1 << 20):
+        """The collected records as (x, y) tuples, `slab` words at a time."""
+        out: list = []
+        if store.failed:
+            raise MemoryError("no memory for the collected records")
+        if not store.len:
+            return out
+        words = np.frombuffer((ctypes.c_uint32 * store.len).from_address(store.data), np.uint32)
+        at = 0
+        while at < words.size:
+            w = words[at:at + slab].tolist()
+            i, m = 0, len(w)
+            while i + 2 <= m:
+                j = i + 2 + w[i]
+                e = j + w[i + 1]
+                if e > m:
+                    break
+                out.append((tuple(w[i + 2:j]), tuple(w[j:e])))
+                i = e
+            if i == 0:
+                slab *= 2       # (a record longer than the slab)
+            at += i
+        return out
 
     @staticmethod
     def _stats(st, results):
@@ -376,22 +407,25 @@ class Graph:
                 task_buf[i] = _Task(r, f, l, 0, 0.0)
             o.tasks = ctypes.cast(task_buf, ctypes.c_void_p)
             o.n_tasks = len(rows)
-        out: list = []
-        cb = self._sink(collect, sink, out)
+        store = _Collector()
+        cb, user = self._sink(collect, sink, store)
         o.emit = 1 if (collect or sink is not None) else 0
         o.out_words = out_words
         st = _Stats()
-        while True:
-            out.clear()
-            rc = lib.gmk_enumerate(self._h, ctypes.byref(o), cb, None, ctypes.byref(st))
-            # a record buffer overflow is retried with a larger buffer only when
-            # no caller sink has seen results yet
-            if rc != E_OUTBUF or sink is not None:
-                break
-            o.out_words = (o.out_words or (64 << 20)) * 4
-        if rc != E_SINK:
-            _check(rc)
-        return self._stats(st, out if collect else None)
+        try:
+            while True:
+                store.len = 0
+                rc = lib.gmk_enumerate(self._h, ctypes.byref(o), cb, user, ctypes.byref(st))
+                # a record buffer overflow is retried with a larger buffer only when
+                # no caller sink has seen results yet
+                if rc != E_OUTBUF or sink is not None:
+                    break
+                o.out_words = (o.out_words or (64 << 20)) * 4
+            if rc != E_SINK:
+                _check(rc)
+            return self._stats(st, self._records(store) if collect else None)
+        finally:
+            lib.gmk_collect_free(ctypes.byref(store))
 
     def enumerate_resumable(self, checkpoint: str, batch_roots: int = 0, max_batches: int = 0,
                             k: int = 1, result_limit: int = 0, schedule: str = "batched",
@@ -407,14 +441,17 @@ class Graph:
                               tuning.get("pair_limit", 0), task_cost, tuning.get("shard", 0),
                               tuning.get("nshards", 1), engine, tuning.get("split_min_nodes", 0),
                               0, 0)
-        out: list = []
-        cb = self._sink(collect, sink, out)
+        store = _Collector()
+        cb, user = self._sink(collect, sink, store)
         o.emit = 1 if (collect or sink is not None) else 0
         if o.emit:
             o.out_words = tuning.get("out_words", 0)
         st = _Stats()
-        rc = lib.gmk_enumerate_resumable(self._h, ctypes.byref(o), os.fsencode(checkpoint),
-                                         batch_roots, max_batches, cb, None, ctypes.byref(st))
-        if rc not in (0, PAUSED, E_SINK):
-            _check(rc)
-        return self._stats(st, out if collect else None), rc == PAUSED
+        try:
+            rc = lib.gmk_enumerate_resumable(self._h, ctypes.byref(o), os.fsencode(checkpoint),
+                                             batch_roots, max_batches, cb, user, ctypes.byref(st))
+            if rc not in (0, PAUSED, E_SINK):
+                _check(rc)
+            return self._stats(st, self._records(store) if collect else None), rc == PAUSED
+        finally:
+            lib.gmk_collect_free(ctypes.byref(store))
