@@ -139,4 +139,5 @@ def test_fans_of_children(nu, nv, m, k):
             assert dg.enumerate(k=k, **kw).summary() == want, kw
         st = dg.enumerate(k=k, result_limit=want[0] // 2)
         assert st.count == want[0] // 2 and st.truncated
-        assert [s.summary() for s in G.enumerate_batch([dg, dg], [k, k])] == [want, want]
+        with G.Graph.from_graph(g) as other:
+            assert [s.summary() for s in G.enumerate_batch([dg, other], [k, k])] == [want, want]
