@@ -80,7 +80,8 @@ void gmk_graph_free(gmk_graph* g);
  * first-level children). */
 enum {
     GMK_SCHEDULE_PLAIN = 0,    /* one task per root, roots in id order (largest task_cost
-                                  first when one is given), no splitting */
+                                  first when one is given), no splitting,
+                                  children built one by one */
     GMK_SCHEDULE_BATCHED = 1,  /* roots split into chunks, persistent work queue; unfinished
                                   search trees are split into the next round's tasks */
     GMK_SCHEDULE_ORDERED = 2   /* batched over planned tasks: roots split into chunks in
@@ -154,7 +155,8 @@ typedef struct {
                                  its hashes may include results past the limit and are not a
                                  summary of any particular `count` results; emit = 1 runs hash
                                  exactly the delivered results. */
-    uint64_t nodes;           /* search-tree nodes */
+    uint64_t nodes;           /* search-tree nodes (a node whose undecided sets are all tested
+                                 at once counts its k-biplex subsets) */
     uint64_t algo_bytes;      /* adjacency/counter bytes the search read (4 per word) */
     uint64_t tasks;           /* search tasks in the queue */
     uint64_t tasks_done;      /* tasks taken from the queue */
