@@ -29,6 +29,7 @@
 #include "enum_warp.cuh"
 #include "enum_dense.cuh"
 #include "mlp.cuh"
+#include "workspace.h"
 
 namespace {
 
@@ -571,16 +572,32 @@ enumerate_dense_kernel(const __grid_constant__ DenseArgs a) {
             // (written moments ago by a warp on another SM: L2-coherent loads)
             const uint32_t* r = a.share.rec + ticket * kRecordWords;
             next_gid = kBatch ? __ldcg(r + 1) : 0u;
+            uint32_t u = 0;
             #pragma unroll
             for (int w = 0; w < N; ++w) {
                 s.iu[w] = __ldcg(r + kHeader + w); s.iv[w] = __ldcg(r + kHeader + N + w);
                 s.cu[w] = __ldcg(r + kHeader + 2 * N + w); s.cv[w] = __ldcg(r + kHeader + 3 * N + w);
             }
+            #pragma unroll
+            for (int w = N - 1; w >= 0; --w)
+                if (s.iu[w]) u = 32 * w + __ffs(s.iu[w]);
+            // a record that names no graph or no root of it is reported, never followed
+            bool bad = kBatch && next_gid >= a.n_graphs;
+            bad = bad || u == 0 || u > (kBatch ? a.graphs[next_gid].g.nl : a.single.g.nl);
             if (kFans<N>) {
                 // (with its children: the bottom of this warp's stack)
-                if (lane < entry_words<N>()) stack_at<N>(t, 0)[lane] = __ldcg(r + kHeader + lane);
+                const uint32_t e = lane < entry_words<N>() ? __ldcg(r + kHeader + lane) : 0u;
+                bad = __any_sync(kFull, bad || (lane == 5 * N && e > 2));
+                if (lane < entry_words<N>()) stack_at<N>(t, 0)[lane] = e;
                 have = false;
                 sp = 1;
+            }
+            if (bad) {
+                if (lane == 0) {
+                    atomicCAS(&a.ctr->error, 0, gmk::TASK_E_RECORD);
+                    atomicExch(&a.ctr->stop, 1);
+                }
+                break;
             }
         } else {
             if (lane == 0) atomicAdd(&a.rc->tasks_done, 1ull);
@@ -866,15 +883,14 @@ DeviceInfo g_dev[kMaxDevices];
 
 namespace {
 
-int grow(void** p, size_t* have, size_t need) {
-    if (*have >= need && *p) return GMK_OK;
-    if (*p) cudaFree(*p);
-    *p = nullptr;
-    *have = 0;
-    cudaError_t e = cudaMalloc(p, need);
-    if (e != cudaSuccess) { *p = nullptr; return cuda_fail(e, "cudaMalloc(workspace)"); }
-    *have = need;
-    return GMK_OK;
+int grow(void** p, size_t* have, size_t need, bool* fresh = nullptr) {
+    return gmk::grow_buffer(
+        p, have, need, fresh,
+        [](void** q, size_t bytes) {
+            const cudaError_t e = cudaMalloc(q, bytes);
+            return e == cudaSuccess ? GMK_OK : cuda_fail(e, "cudaMalloc(workspace)");
+        },
+        [](void* q) { cudaFree(q); });
 }
 
 // Per-device cache of graph buffers, streams and events.  Loading and freeing
@@ -1522,14 +1538,16 @@ int run_dense(std::vector<GraphJob>& jobs, const gmk_opts* opts, int words, Work
     if (opts->schedule != GMK_SCHEDULE_PLAIN) {
         const uint64_t slots = std::max<uint64_t>(1ull << 16, workers * 128ull);
         const size_t need = slots * gmk::dense::kRecordWords * 4;
-        const void* had = ws.d_states;
-        if ((rc = grow((void**)&ws.d_states, &ws.states_bytes, need))) return rc;
         // a record counts when it carries this launch's number; a new buffer,
         // and one whose numbers are used up, starts cleared
-        if (ws.d_states != had || ++ws.dense_launch == 0) {
-            CK(cudaMemsetAsync(ws.d_states, 0, ws.states_bytes, g0->stream));
-            ws.dense_launch = 1;
-        }
+        bool fresh = false, clear = false;
+        rc = grow((void**)&ws.d_states, &ws.states_bytes, need, &fresh);
+        if (fresh) ws.dense_launch = 0;
+        if (rc) return rc;
+        const uint32_t launch = gmk::next_launch(ws.dense_launch, 0xFFFFFFFFu, &clear);
+        ws.dense_launch = 0;   // (until the clear is queued)
+        if (clear) CK(cudaMemsetAsync(ws.d_states, 0, ws.states_bytes, g0->stream));
+        ws.dense_launch = launch;
         a.share.rec = ws.d_states;
         a.share.slots = (uint32_t)slots;
         a.share.launch = ws.dense_launch;
@@ -1773,11 +1791,11 @@ int run_jobs(std::vector<GraphJob>& jobs, const gmk_opts* opts, gmk_sink sink, v
     if (share) {
         dq_word_cap = std::max<unsigned long long>(1ull << 22, workers * 4096ull);
         dq_idx_cap = std::max<unsigned long long>(1ull << 16, workers * 64ull);
-        const size_t had = ws.dq_idx_bytes;
-        const void* had_p = ws.d_dq_idx;
         if ((rc = grow((void**)&ws.d_dq_words, &ws.dq_words_bytes, dq_word_cap * 4))) return rc;
-        if ((rc = grow((void**)&ws.d_dq_idx, &ws.dq_idx_bytes, dq_idx_cap * 8))) return rc;
-        if (ws.dq_idx_bytes != had || ws.d_dq_idx != had_p) ws.dq_launch = 0;
+        bool fresh = false;
+        rc = grow((void**)&ws.d_dq_idx, &ws.dq_idx_bytes, dq_idx_cap * 8, &fresh);
+        if (fresh) ws.dq_launch = 0;
+        if (rc) return rc;
     }
     const unsigned grid = (unsigned)(threads / block);
     const unsigned long long watchdog_ns = (unsigned long long)opts->watchdog_ms * 1000000ull;
@@ -1874,10 +1892,12 @@ int run_jobs(std::vector<GraphJob>& jobs, const gmk_opts* opts, gmk_sink sink, v
             if (share) {
                 // a slot counts when it carries this launch's number: a new
                 // index, and one whose numbers are used up, starts cleared
-                if (ws.dq_launch == 0 || ++ws.dq_launch >= 1u << (64 - gmk::warp::kTagShift)) {
-                    CK(cudaMemsetAsync(ws.d_dq_idx, 0, ws.dq_idx_bytes, g0->stream));
-                    ws.dq_launch = 1;
-                }
+                bool clear = false;
+                const uint32_t launch =
+                    gmk::next_launch(ws.dq_launch, (1u << (64 - gmk::warp::kTagShift)) - 1, &clear);
+                ws.dq_launch = 0;   // (until the clear is queued)
+                if (clear) CK(cudaMemsetAsync(ws.d_dq_idx, 0, ws.dq_idx_bytes, g0->stream));
+                ws.dq_launch = launch;
                 a.share.tag = (unsigned long long)ws.dq_launch << gmk::warp::kTagShift;
             }
             warp_kernel(which)<<<grid, kWBlock, 0, g0->stream>>>(a);
