@@ -30,7 +30,8 @@
 //
 // States waiting on the warp's stack are handed to idle warps (tickets and
 // slots, as in the list-based kernel; a record is one stack entry, and its slot
-// holds it, so there is no separate index).
+// holds it, so there is no separate index).  Slots are used again (state_ring.h):
+// a search of any length stays shared to its end.
 //
 // What bounds it: integer issue, and on graphs of a few thousand nodes the
 // latency of one warp's chain of nodes.  The list-based search of the same
@@ -43,6 +44,7 @@
 // 10.4 -> 2.2.
 #pragma once
 #include "enum_warp.cuh"
+#include "state_ring.h"
 
 namespace gmk {
 namespace dense {
@@ -58,11 +60,11 @@ constexpr uint32_t kMinShare = 10;     // candidates of a state worth handing on
 // 1.3x faster than 4 at k = 1 (16: 1.35x, but 1.4x slower at k = 3); with more
 // mask words a node costs more, and 4 is 5-10 % faster than 2 or 8.
 template <int N> __host__ __device__ constexpr uint32_t poll_nodes() { return N == 1 ? 8 : 4; }
-constexpr uint32_t kShareMax = 8;      // states handed on per look, at most
-// A record: launch number (written last), graph, 2 spare words, a state.  All
-// N use one record size: a record is recognised by the launch number in its
-// first word, which must never have been another launch's state word.
+// A record: mark (written last), graph, 2 spare words, a state.  All N use one
+// record size: a record is recognised by the mark in its first word, which must
+// never have been another launch's state word.
 constexpr uint32_t kHeader = 4;
+constexpr unsigned long long kRingLimitNs = 10000000000ull;   // a slot not read for 10 s: an error
 constexpr uint32_t kRecordWords = kHeader + 21;
 // Stack entries in shared memory; deeper ones are in the warp's global spill
 // area.  One entry per included candidate on the path (a fan leaves one for all
@@ -99,15 +101,15 @@ struct Shared {
 };
 
 struct Share {
-    uint32_t* rec;                    // fixed-size records, slot t for ticket t
-    uint32_t slots;
-    uint32_t launch;                  // a record is valid when its first word is this number
-    unsigned long long* tail;         // slots reserved
+    uint32_t* rec;                    // fixed-size records, one per slot of the ring
+    StateRing ring;
+    unsigned long long* tail;         // tickets reserved
     unsigned long long* claim;        // tickets taken by waiting warps
     unsigned long long* outstanding;  // unfinished tasks - queue_len (mod 2^64)
     unsigned long long* donated;
-    int* full;
     int* done;                        // warp::kDoneFlags flags, as warp::Donation's
+    int* stop;                        // the launch's stop and error words
+    int* error;
     uint32_t min_nodes;
 };
 
@@ -518,14 +520,52 @@ __device__ __forceinline__ bool node(Ctx<N>& t, State<N>& s, bool fit) {
     return false;
 }
 
+// Tickets that wait for a record (lane 0), at most 32; kWantChecked in it: they
+// are to be counted again (waiting_now) before any is served.
+constexpr uint32_t kWantChecked = 64;
+__device__ __forceinline__ uint32_t waiting(const Share& sh) {
+    const unsigned long long tail = *(volatile const unsigned long long*)sh.tail;
+    const long long w = (long long)(*(volatile const unsigned long long*)sh.claim - tail);
+    return w <= 0 ? 0u : (uint32_t)(w < 32 ? w : 32) | (sh.ring.early(tail) ? 0u : kWantChecked);
+}
+// The same as of one moment: the claimed tickets are read before the reserved ones.
+__device__ __forceinline__ uint32_t waiting_now(const Share& sh) {
+    unsigned long long claim;
+    asm volatile("ld.acquire.gpu.u64 %0, [%1];" : "=l"(claim) : "l"(sh.claim) : "memory");
+    const long long w = (long long)(claim - *(volatile const unsigned long long*)sh.tail);
+    return w > 0 ? (uint32_t)(w < 32 ? w : 32) : 0u;
+}
+
+// Waits until the slot r of `ticket` has been read by its last user (a warp that
+// runs: one look, as a rule).  False: the launch stops, or the wait ran out.
+__device__ __forceinline__ bool ring_wait(const Share& sh, unsigned long long ticket, const uint32_t* r) {
+    if (sh.ring.first(ticket)) return true;
+    unsigned long long since = 0;
+    #pragma unroll 1
+    for (uint32_t spin = 0; !sh.ring.free(ticket, *(volatile const uint32_t*)r); ++spin) {
+        if (load_flag(sh.stop)) return false;
+        const unsigned long long now = now_ns();
+        if (spin == 0) since = now;
+        if (now - since > kRingLimitNs) {
+            atomicCAS(sh.error, 0, TASK_E_TIMEOUT);
+            atomicExch(sh.stop, 1);
+            return false;
+        }
+        __nanosleep(64);
+    }
+    return true;       // (the caller's stores wait for the branch)
+}
+
 // Hands up to `want` of the oldest entries (those with kMinShare candidates
 // and children or more) to waiting warps.
 template <int N>
 __device__ __forceinline__ void donate(Ctx<N>& t, const Share& sh, uint32_t gid, uint32_t want) {
     __syncwarp();
+    const bool checked = want & kWantChecked;
+    want &= kWantChecked - 1;
     uint32_t n = t.sp - t.bottom;
     n = n < want ? n : want;
-    n = n < kShareMax ? n : kShareMax;
+    n = n < kRingShare ? n : kRingShare;
     // lane i < n: the i-th oldest; the run of large ones from the bottom
     uint32_t c = 0;
     if (t.lane < n) {
@@ -538,31 +578,32 @@ __device__ __forceinline__ void donate(Ctx<N>& t, const Share& sh, uint32_t gid,
         }
     }
     const uint32_t small = __ballot_sync(kFull, t.lane >= n || c < kMinShare);
-    n = __ffs(small) - 1;      // (n <= kShareMax < 32: some lane is set)
+    n = __ffs(small) - 1;      // (n <= kRingShare < 32: some lane is set)
     if (n == 0) return;
-    unsigned long long slot = 0;
-    int ok = 0;
+    if (checked) {
+        want = bcast(waiting_now(sh));
+        n = n < want ? n : want;
+        if (n == 0) return;
+    }
+    unsigned long long ticket = 0;
     if (t.lane == 0) {
-        slot = atomicAdd(sh.tail, (unsigned long long)n);
-        ok = slot + n <= sh.slots;
-        if (ok) {
-            atomicAdd(sh.outstanding, (unsigned long long)n);   // before they can finish
-            atomicAdd(sh.donated, (unsigned long long)n);
-        } else {
-            atomicExch(sh.full, 1);
+        ticket = atomicAdd(sh.tail, (unsigned long long)n);
+        atomicAdd(sh.outstanding, (unsigned long long)n);   // before they can finish
+        atomicAdd(sh.donated, (unsigned long long)n);
+    }
+    ticket = bcast(ticket) + t.lane;
+    if (t.lane < n) {
+        uint32_t* r = sh.rec + (unsigned long long)sh.ring.slot(ticket) * kRecordWords;
+        if (ring_wait(sh, ticket, r)) {
+            const uint32_t* e = stack_at<N>(t, t.bottom + t.lane);
+            r[1] = gid;
+            #pragma unroll
+            for (uint32_t w = 0; w < entry_words<N>(); ++w) r[kHeader + w] = e[w];
+            __threadfence();
+            atomicExch(r, sh.ring.ready(ticket));
         }
     }
-    if (!bcast(ok)) return;
-    slot = bcast(slot);
-    uint32_t* r = sh.rec + (slot + t.lane) * kRecordWords;
-    if (t.lane < n) {
-        const uint32_t* e = stack_at<N>(t, t.bottom + t.lane);
-        r[1] = gid;
-        #pragma unroll
-        for (uint32_t w = 0; w < entry_words<N>(); ++w) r[kHeader + w] = e[w];
-        __threadfence();
-        atomicExch(r, sh.launch);
-    }
+    __syncwarp();
     t.bottom += n;
     __syncwarp();
 }

@@ -536,12 +536,14 @@ enumerate_dense_kernel(const __grid_constant__ DenseArgs a) {
             unsigned long long ticket = 0;
             if (lane == 0) {
                 ticket = atomicAdd(a.share.claim, 1ull);
-                const volatile uint32_t* slot = a.share.rec + ticket * kRecordWords;
+                const volatile uint32_t* slot =
+                    a.share.rec + (unsigned long long)a.share.ring.slot(ticket) * kRecordWords;
+                const uint32_t ready = a.share.ring.ready(ticket);
                 const volatile int* done = a.share.done + (blockIdx.x % gmk::warp::kDoneFlags) * 32;
                 unsigned long long seen = ~0ull, t_seen = gmk::now_ns();
                 unsigned sleep_ns = 32;
                 for (uint32_t spin = 0;; ++spin) {
-                    if (ticket < a.share.slots && *slot == a.share.launch) break;
+                    if (*slot == ready) break;
                     if (*done) { quit = 1; break; }
                     if ((spin & 7u) == 7u && gmk::load_flag(&a.ctr->stop)) { quit = 1; break; }
                     if ((spin & 63u) == 0) {
@@ -570,13 +572,14 @@ enumerate_dense_kernel(const __grid_constant__ DenseArgs a) {
             if (quit) break;
             ticket = bcast(ticket);
             // (written moments ago by a warp on another SM: L2-coherent loads)
-            const uint32_t* r = a.share.rec + ticket * kRecordWords;
+            uint32_t* r = a.share.rec + (unsigned long long)a.share.ring.slot(ticket) * kRecordWords;
             next_gid = kBatch ? __ldcg(r + 1) : 0u;
-            uint32_t u = 0;
+            uint32_t u = 0, got = next_gid;
             #pragma unroll
             for (int w = 0; w < N; ++w) {
                 s.iu[w] = __ldcg(r + kHeader + w); s.iv[w] = __ldcg(r + kHeader + N + w);
                 s.cu[w] = __ldcg(r + kHeader + 2 * N + w); s.cv[w] = __ldcg(r + kHeader + 3 * N + w);
+                got |= s.iu[w] | s.iv[w] | s.cu[w] | s.cv[w];
             }
             #pragma unroll
             for (int w = N - 1; w >= 0; --w)
@@ -589,9 +592,15 @@ enumerate_dense_kernel(const __grid_constant__ DenseArgs a) {
                 const uint32_t e = lane < entry_words<N>() ? __ldcg(r + kHeader + lane) : 0u;
                 bad = __any_sync(kFull, bad || (lane == 5 * N && e > 2));
                 if (lane < entry_words<N>()) stack_at<N>(t, 0)[lane] = e;
+                got |= e;
                 have = false;
                 sp = 1;
             }
+            // read: the slot is free.  The store is decided by the loaded words (a
+            // state has a root), so they have arrived when it is issued; a fence
+            // here would hold every shared state up (58 x 58, k = 2: 2.6 -> 2.8 ms)
+            got = __reduce_or_sync(kFull, got);
+            if (lane == 0 && got) *(volatile uint32_t*)r = a.share.ring.ready(ticket) + 1;
             if (bad) {
                 if (lane == 0) {
                     atomicCAS(&a.ctr->error, 0, gmk::TASK_E_RECORD);
@@ -674,15 +683,12 @@ enumerate_dense_kernel(const __grid_constant__ DenseArgs a) {
             }
             if (++polls == poll_nodes<N>()) {
                 polls = 0;
-                int late = 0, want = 0, done = 0;
+                int late = 0, done = 0;
+                uint32_t want = 0;
                 if (lane == 0) {
                     done = gmk::load_flag(&a.ctr->stop) || (kBatch && gmk::load_flag(&ctr->stop));
                     late = deadline && gmk::now_ns() > deadline;
-                    if (share && nodes >= a.share.min_nodes && t.sp != t.bottom && !gmk::load_flag(a.share.full)) {
-                        const long long w = (long long)(*(volatile const unsigned long long*)a.share.claim -
-                                                        *(volatile const unsigned long long*)a.share.tail);
-                        want = w > 0 ? (int)(w < 32 ? w : 32) : 0;
-                    }
+                    if (share && nodes >= a.share.min_nodes && t.sp != t.bottom) want = waiting(a.share);
                 }
                 done = bcast(done); late = bcast(late); want = bcast(want);
                 if (late && lane == 0) {
@@ -690,7 +696,7 @@ enumerate_dense_kernel(const __grid_constant__ DenseArgs a) {
                     atomicExch(&a.ctr->stop, 1);
                 }
                 if (done || late) { quit = true; break; }
-                if (want) donate<N>(t, a.share, gid, (uint32_t)want);
+                if (want) donate<N>(t, a.share, gid, want);
                 if (limit && t.cnt >= gmk::kFlushBatch) flush();
             }
             ++nodes;
@@ -849,14 +855,14 @@ struct Workspace {
     unsigned long long* d_dq_idx = nullptr;
     size_t dq_idx_bytes = 0;
     uint32_t dq_launch = 0;       // the last launch's number; 0: the index is not cleared yet
-    // small graphs' search: stack spill, records of shared states (each valid for
-    // the launch whose number it carries), counters of a launch and their pinned
-    // copy on the host
+    // small graphs' search: stack spill, the ring of shared states and its next
+    // mark (0: to be cleared), counters of a launch and their pinned copy on the
+    // host
     uint32_t* d_spill = nullptr;
     size_t spill_bytes = 0;
     uint32_t* d_states = nullptr;
     size_t states_bytes = 0;
-    uint32_t dense_launch = 0;
+    uint32_t state_marks = 0;
     void* d_dense = nullptr;
     size_t dense_bytes = 0;
     void* h_dense = nullptr;
@@ -1536,27 +1542,25 @@ int run_dense(std::vector<GraphJob>& jobs, const gmk_opts* opts, int words, Work
     DenseArgs a;
     std::memset(&a, 0, sizeof(a));
     if (opts->schedule != GMK_SCHEDULE_PLAIN) {
-        const uint64_t slots = std::max<uint64_t>(1ull << 16, workers * 128ull);
-        const size_t need = slots * gmk::dense::kRecordWords * 4;
-        // a record counts when it carries this launch's number; a new buffer,
-        // and one whose numbers are used up, starts cleared
+        // a slot counts by its mark; a new buffer, and one whose marks are used
+        // up, starts cleared
         bool fresh = false, clear = false;
+        const uint64_t running = std::min(workers, resident);
+        const size_t need = gmk::ring_begin(running, 0, &clear).slots() * (size_t)gmk::dense::kRecordWords * 4;
         rc = grow((void**)&ws.d_states, &ws.states_bytes, need, &fresh);
-        if (fresh) ws.dense_launch = 0;
+        if (fresh) ws.state_marks = 0;
         if (rc) return rc;
-        const uint32_t launch = gmk::next_launch(ws.dense_launch, 0xFFFFFFFFu, &clear);
-        ws.dense_launch = 0;   // (until the clear is queued)
+        a.share.ring = gmk::ring_begin(running, ws.state_marks, &clear);
+        ws.state_marks = 0;   // (until the launch is over and its tickets are known)
         if (clear) CK(cudaMemsetAsync(ws.d_states, 0, ws.states_bytes, g0->stream));
-        ws.dense_launch = launch;
         a.share.rec = ws.d_states;
-        a.share.slots = (uint32_t)slots;
-        a.share.launch = ws.dense_launch;
         a.share.tail = &dc->rc.dq_tail;
         a.share.claim = &dc->rc.dq_claim;
         a.share.outstanding = &dc->rc.outstanding;
         a.share.donated = &dc->rc.donated;
-        a.share.full = &dc->rc.dq_full;
         a.share.done = &dc->rc.done[0][0];
+        a.share.stop = &dc->launch.stop;
+        a.share.error = &dc->launch.error;
         a.share.min_nodes = opts->donate_min_nodes ? opts->donate_min_nodes : kDenseDonateMin;
     }
     a.single = gt[0];
@@ -1581,6 +1585,7 @@ int run_dense(std::vector<GraphJob>& jobs, const gmk_opts* opts, int words, Work
     CK(cudaMemcpyAsync(ws.h_dense, dc, ctr_bytes, cudaMemcpyDeviceToHost, g0->stream));
     CK(cudaStreamSynchronize(g0->stream));
     const DenseCounters* h = static_cast<const DenseCounters*>(ws.h_dense);
+    if (a.share.rec) ws.state_marks = gmk::ring_next(a.share.ring, h->rc.dq_tail);
     for (size_t i = 0; i < ng; ++i) {
         if (!jobs[i].root_nodes) continue;
         gmk_graph* g = jobs[i].g;

@@ -1,12 +1,14 @@
 """Sharing of search states between the warps of the small graphs' search: runs
-that make its workspace grow, in a process of their own, so that the workspace
-starts empty."""
+that make its workspace grow (in a process of their own, so that the workspace
+starts empty), and runs that hand on more states than there are slots for."""
 import os
 import subprocess
 import sys
 
 import pytest
 
+import gmkbe_b200 as G
+from gmkbe_b200 import graphgen as gg
 from conftest import ROOT
 
 pytestmark = pytest.mark.gpu
@@ -41,3 +43,15 @@ def test_runs_that_grow_the_workspace():
                          env=dict(os.environ, PYTHONPATH=ROOT + os.pathsep + os.path.join(ROOT, "tests")),
                          timeout=300)
     assert out.returncode == 0 and out.stdout.strip() == "ok", out.stderr[-2000:]
+
+
+@pytest.mark.parametrize("nu,nv,p", [(80, 80, 0.35), (64, 60, 0.5)])
+def test_states_handed_on_past_the_last_slot(nu, nv, p):
+    # 64 slots a warp, rounded up to a power of two: the tickets go past the last
+    # slot, and the next launch starts from the marks that this one left
+    with G.Graph.from_graph(gg.erdos_renyi(nu, nv, p, 3)) as dg:
+        want = dg.enumerate(k=1, sharing=False).summary()
+        for _ in range(2):
+            st = dg.enumerate(k=1, watchdog_ms=60_000)
+            assert st.summary() == want
+            assert st.donations > 1 << (64 * (st.threads // 32) - 1).bit_length()
