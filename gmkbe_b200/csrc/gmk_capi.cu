@@ -1254,9 +1254,11 @@ std::vector<uint32_t> select_roots(uint32_t nl, const float* cost, uint32_t rb, 
     return std::vector<uint32_t>(order.begin() + rb, order.begin() + re);
 }
 
-// Narrowest chunk of first-level children: of gmk_plan_tasks, and of the
-// tasks that a run of the list-based kernel makes itself -- its children are
-// looked at 32 at a time.
+// Narrowest chunk of first-level children: of gmk_plan_tasks and of the thread
+// engine's tasks, and of the tasks that a run of the list-based kernel makes itself
+// -- that one looks at its children 32 at a time.  (The thread engine never
+// splits a task, so its tail is its widest one: er200, k = 1 takes 1.60 s with 16
+// and 3.95 s with 64.)
 constexpr uint32_t kPlanChunk = 16;
 constexpr uint32_t kMinChunk = 64;
 
@@ -1712,7 +1714,8 @@ int run_jobs(std::vector<GraphJob>& jobs, const gmk_opts* opts, gmk_sink sink, v
     const bool planned = is_planned(jobs, opts);
     std::vector<gmk_task> plan;
     const uint32_t max_chunks = opts->schedule == GMK_SCHEDULE_PLAIN ? 1u : 0xFFFFFFFFu;
-    if (planned && (rc = plan_jobs(jobs, opts, workers, max_chunks, kMinChunk, plan))) return rc;
+    const uint32_t min_chunk = warp ? kMinChunk : kPlanChunk;
+    if (planned && (rc = plan_jobs(jobs, opts, workers, max_chunks, min_chunk, plan))) return rc;
     unsigned long long n_tasks = 0;
     for (size_t i = 0; i < ng; ++i) {
         const GraphJob& j = jobs[i];
@@ -1724,10 +1727,10 @@ int run_jobs(std::vector<GraphJob>& jobs, const gmk_opts* opts, gmk_sink sink, v
             if (opts->chunk) {
                 chunk = std::min(opts->chunk, nv);
             } else {
-                // about tasks_per (8) tasks per worker, but no chunk below kMinChunk children
+                // about tasks_per (8) tasks per worker, but no chunk below min_chunk children
                 const uint64_t want = (uint64_t)tasks_per * workers;
                 const uint64_t per_root = (want + g->nl - 1) / std::max<uint32_t>(g->nl, 1);
-                chunk = (uint32_t)std::max<uint64_t>(kMinChunk, (nv + per_root - 1) / std::max<uint64_t>(1, per_root));
+                chunk = (uint32_t)std::max<uint64_t>(min_chunk, (nv + per_root - 1) / std::max<uint64_t>(1, per_root));
                 chunk = std::min(chunk, nv);
             }
         }
