@@ -1342,12 +1342,24 @@ bool is_planned(const std::vector<GraphJob>& jobs, const gmk_opts* opts) {
            (opts->schedule == GMK_SCHEDULE_PLAIN && jobs[0].task_cost);
 }
 
+// Warps per SM that the warp engine's shards are planned for.  Every shard must
+// come from one plan, whatever its rank is asked for, so a sharded run plans for
+// this number and kPlanChunk, not for the kernel that it goes to: that depends on
+// the mode (counts or records), on options and on the build, as its warps per SM
+// and its own chunk width do.  (28: what the checkpoints of sharded runs were
+// written under.)
+constexpr uint32_t kShardWarps = 28;
+
 // The planned tasks of a run for `workers` workers, at most max_chunks a root.
-int plan_jobs(std::vector<GraphJob>& jobs, const gmk_opts* opts, uint64_t workers,
+int plan_jobs(std::vector<GraphJob>& jobs, const gmk_opts* opts, int sms, uint64_t workers,
               uint32_t max_chunks, uint32_t min_width, std::vector<gmk_task>& plan) {
     int rc;
     const size_t ng = jobs.size();
     const uint32_t nsh = opts->nshards > 1 ? opts->nshards : 1u;
+    if (nsh > 1 && opts->engine == GMK_ENGINE_WARP) {
+        workers = opts->threads ? std::max<uint64_t>(1, opts->threads / 32) : (uint64_t)sms * kShardWarps;
+        min_width = kPlanChunk;
+    }
     const uint32_t sh = nsh > 1 ? opts->shard : 0u;
     const uint32_t tasks_per = opts->tasks_per_worker ? opts->tasks_per_worker : 8u;
     if (opts->tasks) {
@@ -1491,7 +1503,7 @@ int run_dense(std::vector<GraphJob>& jobs, const gmk_opts* opts, int words, Work
     const bool planned = is_planned(jobs, opts);
     const uint32_t max_chunks = opts->schedule == GMK_SCHEDULE_PLAIN ? 1u : 0xFFFFFFFFu;
     if (planned) {
-        if ((rc = plan_jobs(jobs, opts, workers, max_chunks, kPlanChunk, plan))) return rc;
+        if ((rc = plan_jobs(jobs, opts, di.sms, workers, max_chunks, kPlanChunk, plan))) return rc;
         if ((rc = upload_plan(ws, g0, plan))) return rc;
     }
     const size_t ctr_bytes = sizeof(DenseCounters) + (ng > 1 ? (ng - 1) * sizeof(Counters) : 0);
@@ -1715,7 +1727,7 @@ int run_jobs(std::vector<GraphJob>& jobs, const gmk_opts* opts, gmk_sink sink, v
     std::vector<gmk_task> plan;
     const uint32_t max_chunks = opts->schedule == GMK_SCHEDULE_PLAIN ? 1u : 0xFFFFFFFFu;
     const uint32_t min_chunk = warp ? kMinChunk : kPlanChunk;
-    if (planned && (rc = plan_jobs(jobs, opts, workers, max_chunks, min_chunk, plan))) return rc;
+    if (planned && (rc = plan_jobs(jobs, opts, di.sms, workers, max_chunks, min_chunk, plan))) return rc;
     unsigned long long n_tasks = 0;
     for (size_t i = 0; i < ng; ++i) {
         const GraphJob& j = jobs[i];

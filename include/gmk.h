@@ -117,7 +117,12 @@ typedef struct {
                                  (|S|+|C_U|)*(|S|+|C_V|) <= pair_limit; 0 = 4096 */
     uint32_t shard, nshards;  /* one GPU of several: run only this shard's tasks of the
                                  longest-processing-time partition of gmk_plan_tasks (costs:
-                                 task_cost, else gmk_root_costs); nshards 0 or 1 = all */
+                                 task_cost, else gmk_root_costs; warp engine: tasks_per_worker
+                                 tasks for every warp of threads, or for 28 warps per SM);
+                                 nshards 0 or 1 = all.  The partition depends on the graph, the
+                                 costs, the schedule, threads, tasks_per_worker, the root range
+                                 and the GPU's SM count, on nothing else: shards may differ in
+                                 emit and in the other options */
     int32_t engine;           /* GMK_ENGINE_* */
     uint32_t split_min_nodes; /* warp engine, batched/ordered: a task is split only after this
                                  many nodes; 0 = 64 */
@@ -307,7 +312,8 @@ typedef struct gmk_task_ {
  * common neighbour.  Computed on the graph's device once and cached. */
 int gmk_root_costs(gmk_graph* g, float* out);
 
-/* Host-only planner, the one the ordered schedule and sharding use.  The roots
+/* Host-only planner, the one that sharding uses (and, with chunks at least 64
+ * children wide, the ordered schedule of a run that is not sharded).  The roots
  * at positions [root_begin, root_end) of the cost order (largest first, ties
  * by id) are each split into ceil(cost / unit) chunks of their first-level V
  * children (unit = total cost / target_tasks; at most max_chunks per root,
