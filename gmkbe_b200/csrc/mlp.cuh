@@ -142,16 +142,36 @@ __device__ __forceinline__ void product(const float (*left)[PL], const float (*r
     }
 }
 
+// The same where an operand may be infinite or NaN: a term whose left factor (kBoth:
+// either factor) is zero is left out, as a unit that is off contributes nothing.
+template <int K, bool kBoth, int PL, int PR>
+__device__ __forceinline__ void product_of_nonzeros(const float (*left)[PL], const float (*right)[PR], int ty,
+                                                 int tx, float (&acc)[4][4]) {
+    #pragma unroll 1
+    for (int k = 0; k < K; ++k) {
+        #pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            #pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                const float l = left[k][4 * ty + a], r = right[k][4 * tx + b];
+                if (l != 0.f && (!kBoth || r != 0.f)) acc[a][b] = fmaf(l, r, acc[a][b]);
+            }
+        }
+    }
+}
+
 // The tile's hidden layers (h1t, h2t) and outputs; samples past n count as zero
-// inputs.  h2 of this thread's 4 samples x 4 units stays in `h2`.
-__device__ __forceinline__ void forward_tile(TileShared& s, TileGrad* gr, const __half* x, uint32_t first,
+// inputs.  h2 of this thread's 4 samples x 4 units stays in `h2`.  Returns
+// whether this thread met an input or a unit of h1 that is infinite or NaN.
+__device__ __forceinline__ bool forward_tile(TileShared& s, TileGrad* gr, const __half* x, uint32_t first,
                                              uint32_t n, float (&h2)[4][4]) {
     const int ty = threadIdx.x >> 4, tx = threadIdx.x & 15;
+    bool odd = false;
     for (int i = threadIdx.x; i < kTile * F; i += kThreads) {
         const uint32_t at = first + i / F;
         const float v = at < n ? __half2float(x[(uint64_t)at * F + i % F]) : 0.f;
         s.xt[i % F][i / F] = v;
-        if (gr) gr->x[i / F][i % F] = v;
+        if (gr) { gr->x[i / F][i % F] = v; odd |= !isfinite(v); }
     }
     __syncthreads();
     float h1[4][4];
@@ -167,7 +187,7 @@ __device__ __forceinline__ void forward_tile(TileShared& s, TileGrad* gr, const 
         for (int b = 0; b < 4; ++b) {
             const float v = h1[a][b] > 0.f ? h1[a][b] : 0.f;
             s.h1t[4 * tx + b][4 * ty + a] = v;
-            if (gr) gr->h1[4 * ty + a][4 * tx + b] = v;
+            if (gr) { gr->h1[4 * ty + a][4 * tx + b] = v; odd |= !isfinite(v); }
         }
     }
     __syncthreads();
@@ -193,6 +213,7 @@ __device__ __forceinline__ void forward_tile(TileShared& s, TileGrad* gr, const 
         s.out[threadIdx.x] = o;
     }
     __syncthreads();
+    return odd;
 }
 
 // Forward pass.  What bounds it: latency (a few thousand samples are a few
@@ -227,14 +248,19 @@ __global__ void __launch_bounds__(kThreads) gradient_kernel(const __half* w, con
     TileGrad& g = *reinterpret_cast<TileGrad*>(smem + (sizeof(TileShared) + 15) / 16 * 16);
     const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
     load_weights(w, s);
-    for (int i = tid; i < H * H; i += kThreads) g.w2[i / H][i % H] = __half2float(w[OFF_W2 + i]);
+    bool odd_w = false;
+    for (int i = tid; i < H * H; i += kThreads) {
+        const float v = __half2float(w[OFF_W2 + i]);
+        g.w2[i / H][i % H] = v;
+        odd_w |= !isfinite(v);
+    }
     float dw2[4][4] = {}, dw1[4] = {}, dw3[4] = {}, db2[4] = {};   // dw2: [4 ty + a][4 tx + b] = [j][q]
     float db1 = 0.f, db3 = 0.f, loss = 0.f;
     const uint32_t tiles = (n + kTile - 1) / kTile;
     for (uint32_t t = blockIdx.x; t < tiles; t += gridDim.x) {
         const uint32_t first = t * kTile;
         float h2[4][4];
-        forward_tile(s, &g, x, first, n, h2);
+        bool odd = forward_tile(s, &g, x, first, n, h2) || odd_w;
         if (tid < kTile) {
             const float e = first + tid < n ? s.out[tid] - y[first + tid] : 0.f;
             const float d = 2.f * e / (float)n;
@@ -247,19 +273,30 @@ __global__ void __launch_bounds__(kThreads) gradient_kernel(const __half* w, con
         #pragma unroll
         for (int a = 0; a < 4; ++a) {
             const float d = g.dout[4 * ty + a];
+            const bool live = first + 4 * ty + a < n;     // (a sample past n adds nothing)
             #pragma unroll
             for (int b = 0; b < 4; ++b) {
-                dw3[b] = fmaf(d, h2[a][b], dw3[b]);
-                const float v = h2[a][b] > 0.f ? d * s.w3[4 * tx + b] : 0.f;
+                const float h = live ? h2[a][b] : 0.f;
+                dw3[b] = fmaf(d, h, dw3[b]);
+                const float v = h > 0.f ? d * s.w3[4 * tx + b] : 0.f;
+                odd |= !isfinite(v);
                 db2[b] += v;
                 g.dh2[4 * ty + a][4 * tx + b] = v;
                 s.h2t[4 * tx + b][4 * ty + a] = v;
             }
         }
-        __syncthreads();
-        product<kTile>(g.dh2, g.h1, ty, tx, dw2);
+        // a zero times an infinity is NaN, but a unit that is off, or an output that
+        // is right, has no part in the gradient: such a tile (an input past FP16's
+        // range, say) takes its products term by term
+        odd = __syncthreads_or(odd);
         float dh1[4][4] = {};
-        product<H>(s.h2t, g.w2, ty, tx, dh1);
+        if (odd) {
+            product_of_nonzeros<kTile, true>(g.dh2, g.h1, ty, tx, dw2);
+            product_of_nonzeros<H, false>(s.h2t, g.w2, ty, tx, dh1);
+        } else {
+            product<kTile>(g.dh2, g.h1, ty, tx, dw2);
+            product<H>(s.h2t, g.w2, ty, tx, dh1);
+        }
         __syncthreads();   // every thread has read h1
         #pragma unroll
         for (int a = 0; a < 4; ++a) {
@@ -273,6 +310,7 @@ __global__ void __launch_bounds__(kThreads) gradient_kernel(const __half* w, con
         for (int i = 0; i < kTile; ++i) {
             const float d = g.h1[i][tid >> 2];
             const float4 v = *reinterpret_cast<const float4*>(&g.x[i][4 * (tid & 3)]);
+            if (odd && d == 0.f) continue;
             dw1[0] = fmaf(d, v.x, dw1[0]); dw1[1] = fmaf(d, v.y, dw1[1]);
             dw1[2] = fmaf(d, v.z, dw1[2]); dw1[3] = fmaf(d, v.w, dw1[3]);
             if ((tid & 3) == 0) db1 += d;
