@@ -491,7 +491,7 @@ enumerate_dense_kernel(const __grid_constant__ DenseArgs a) {
         }
         deadline = bcast(t0) + a.watchdog_ns;
     }
-    uint32_t gid = 0xFFFFFFFFu;
+    uint32_t gid = 0xFFFFFFFFu, polls = 0;
     unsigned long long limit = a.limit;
     Counters* ctr = nullptr;
     unsigned long long left = 1;   // lane 0: tasks of the launch left after its last one
@@ -657,7 +657,6 @@ enumerate_dense_kernel(const __grid_constant__ DenseArgs a) {
             if (s.iu[w]) root = 32 * w + __ffs(s.iu[w]) - 1;
         t.sp = kFans<N> ? sp : 0;
         t.bottom = t.extra = 0;
-        uint32_t polls = 0;
         unsigned long long nodes = 0;
         bool quit = kBatch && gmk::load_flag(&ctr->stop);   // a capped graph's tasks end at once
         quit = __any_sync(gmk::warp::kFull, quit);
@@ -697,7 +696,7 @@ enumerate_dense_kernel(const __grid_constant__ DenseArgs a) {
                 }
                 if (done || late) { quit = true; break; }
                 if (want) donate<N>(t, a.share, gid, want);
-                if (limit && t.cnt >= gmk::kFlushBatch) flush();
+                if (limit && t.cnt + t.nfound >= gmk::kFlushBatch) flush();
             }
             ++nodes;
             have = fit = node<N>(t, s, fit);
@@ -706,6 +705,9 @@ enumerate_dense_kernel(const __grid_constant__ DenseArgs a) {
             if (!kFans<N> && !have && t.sp != t.bottom) have = !pop<N>(t, s);
         }
         t.nodes += nodes;
+        // a limit sees a task's results when the task ends: thousands of warps with
+        // a few unpublished ones each would run a small graph to its end
+        if (limit && t.cnt + t.nfound) flush();
         if (lane == 0) {
             if (G.root_nodes) atomicAdd(G.root_nodes + root, nodes);
             // this task is finished; the last one of the launch ends the waiting
