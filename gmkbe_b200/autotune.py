@@ -17,7 +17,11 @@ over its values, the others fixed; `passes` rounds):
                  roots' costs, so that bucket's roots are cut into more (or
                  fewer) tasks by the planner -- the chunk size per bucket;
   * tasks_per_worker, donate_min_nodes, pair_limit: the planner's task count,
-                 the in-launch sharing threshold, the node-rule threshold.
+                 the in-launch sharing threshold (0: the kernel's own), the
+                 node-rule threshold.
+The defaults are what a run without any of these options uses.  A graph of at
+most 128 vertices a side goes to its own kernel with them; other values of
+bits_min and pair_limit are rules of the list-based one and take it there.
 None of them changes the result set.  Winners are cached in a JSON file keyed
 by graph fingerprint, k and limit, so a graph is tuned once.
 """
@@ -33,7 +37,7 @@ from .api import Graph
 
 NONE = 0xFFFFFFFF
 DEFAULTS = dict(warps=1.0, hash_load=25, bits_min=64, bucket_scale=(1.0, 1.0, 1.0),
-                tasks_per_worker=8, donate_min_nodes=16, pair_limit=4096)
+                tasks_per_worker=8, donate_min_nodes=0, pair_limit=4096)
 CHOICES = {
     "warps": [0.5, 0.75, 1.0],
     "hash_load": [25, 50, 90],
@@ -41,7 +45,7 @@ CHOICES = {
     "bucket_scale": [(1.0, 1.0, 1.0), (1.0, 2.0, 4.0), (1.0, 4.0, 16.0), (2.0, 1.0, 1.0),
                      (0.5, 1.0, 2.0)],
     "tasks_per_worker": [2, 8, 32],
-    "donate_min_nodes": [4, 16, 64],
+    "donate_min_nodes": [0, 4, 64],
     "pair_limit": [1024, 4096, 16384],
 }
 

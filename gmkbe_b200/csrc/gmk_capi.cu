@@ -1456,12 +1456,13 @@ constexpr uint32_t kDenseChunk = 2;
 // of at most kDenseSide vertices a side (at 128 x 128 it is still 3.7x faster
 // than the list-based search, at four words a mask; eight would not leave a
 // lane registers for them).  Runs that bound the list-based
-// search's memory or rules (arena_words, max_members, pair_limit,
-// bits_min_list) or that ask for splitting into launches (no_sharing) keep it,
-// and so do records.
+// search's memory or rules (arena_words, max_members, a pair_limit or
+// bits_min_list other than the default, given or not) or that ask for splitting
+// into launches (no_sharing) keep it, and so do records.
 int dense_words(const std::vector<GraphJob>& jobs, const gmk_opts* opts) {
     if (opts->engine != GMK_ENGINE_WARP || opts->emit || opts->no_sharing || opts->arena_words ||
-        opts->max_members || opts->pair_limit || opts->bits_min_list)
+        opts->max_members || (opts->pair_limit && opts->pair_limit != kDefaultPairLimit) ||
+        (opts->bits_min_list && opts->bits_min_list != gmk::warp::kBitsMinList))
         return 0;
     uint32_t side = 0;
     for (const GraphJob& j : jobs) side = std::max({side, j.g->nl, j.g->n - j.g->nl});

@@ -92,7 +92,11 @@ enum {
                                   results come) */
 };
 
-/* Search engines (same rules, same result set). */
+/* Search engines (same rules, same result set).  The warp engine has a kernel of
+ * its own for small graphs: a run with emit = 0 over graphs of at most 128 vertices
+ * a side goes to a search on bit masks, in one launch, unless arena_words,
+ * max_members or no_sharing is set, or pair_limit or bits_min_list has another
+ * value than its default; these bound or steer the list-based search. */
 enum {
     GMK_ENGINE_WARP = 0,       /* one task per warp, lanes share each node's work (default) */
     GMK_ENGINE_THREAD = 1      /* one task per thread, no splitting */
@@ -103,7 +107,8 @@ typedef struct {
     uint64_t result_limit;    /* -r: stop after this many results; 0 = enumerate all */
     int32_t schedule;         /* GMK_SCHEDULE_* */
     int32_t emit;             /* 0: count + set hash only; 1: also deliver every result to the sink */
-    uint32_t chunk;           /* first-level children per task (batched); 0 = automatic */
+    uint32_t chunk;           /* first-level children per task (batched); 0 = automatic
+                                 (small graphs: 2) */
     uint32_t threads;         /* resident search threads; 0 = automatic */
     uint32_t arena_words;     /* per-thread search arena (u32 words); 0 = automatic */
     uint32_t max_members;     /* largest |X|+|Y| a task may hold; 0 = the bound
@@ -125,7 +130,7 @@ typedef struct {
                                  emit and in the other options */
     int32_t engine;           /* GMK_ENGINE_* */
     uint32_t split_min_nodes; /* warp engine, batched/ordered: a task is split only after this
-                                 many nodes; 0 = 64 */
+                                 many nodes; 0 = 64.  Small graphs: no effect (one launch) */
     uint32_t root_begin;      /* only roots at positions [root_begin, root_end) of the root
                                  order (id order, or cost order for ORDERED); the ranges of */
     uint32_t root_end;        /* consecutive calls partition the result set; root_end 0 = all.
@@ -136,7 +141,7 @@ typedef struct {
     uint32_t donate_min_nodes; /* warp engine, batched/ordered, emit = 0: in-launch work
                                  sharing -- a busy task that has run this many nodes gives the
                                  shallowest unexplored part of its tree to an idle warp;
-                                 0 = 16 */
+                                 0 = 16 (small graphs: 1) */
     int32_t no_sharing;       /* 1: no in-launch sharing (unfinished trees only split into the
                                  next launch, as emit = 1 runs do) */
     const struct gmk_task_* tasks; /* optional explicit task list (gmk_task, e.g. from
@@ -144,7 +149,8 @@ typedef struct {
                                  instead of planning; needs nshards <= 1, no root range,
                                  and one graph.  Used to re-run a failed rank's shard. */
     uint64_t n_tasks;         /* entries of tasks */
-    uint32_t tasks_per_worker; /* batched / ordered: root tasks planned per warp; 0 = 8 */
+    uint32_t tasks_per_worker; /* batched / ordered: root tasks planned per warp; 0 = 8.  Small
+                                 graphs: ordered and sharded runs only */
     uint32_t bits_min_list;   /* warp engine, k >= 2: the intersection strategy by list length --
                                  a branching node's candidate lists of at least this many entries
                                  get filter bitmaps (bit tests), shorter ones are filtered by
