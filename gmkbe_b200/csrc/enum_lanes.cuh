@@ -176,8 +176,10 @@ __device__ __forceinline__ void lane_record(uint32_t* r, const uint32_t* ids, ui
 // on or the lists have been overwritten), or up to kLaneBlocks blocks of 32
 // from h.pos, the last one the first with a child that does not fit.  Writes the
 // frame's position and pending children; *nodes receives the children decided here.
+// False: no block was looked at, the side's children are built one by one from
+// here on (FL_ONE0 / FL_ONE1).
 template <bool kRec>
-__device__ __forceinline__ void lane_blocks(Ctx& t, const Outputs& o, uint32_t cur, const Hdr& h, int s,
+__device__ __forceinline__ bool lane_blocks(Ctx& t, const Outputs& o, uint32_t cur, const Hdr& h, int s,
                                             bool opp_done, LaneCtx& lc, uint32_t* nodes) {
     const GraphView& g = t.g;
     const uint32_t lane = t.lane, k = t.k;
@@ -192,7 +194,7 @@ __device__ __forceinline__ void lane_blocks(Ctx& t, const Outputs& o, uint32_t c
     if (again || lc.cur != cur || lc.next != pos) {
         // the members, one per lane
         pop_to(t, ns);
-        fits = ns <= 15 && k <= 9;
+        fits = ns <= kLaneMembers && k <= kLaneK;
         const bool is_m = fits && lane < ns;
         const uint32_t mid = is_m ? t.sid[lane] : 0u, msc = is_m ? t.smc[lane] : 0u;
         const bool mo = is_m && side_of(g, mid) != s;
@@ -266,6 +268,14 @@ __device__ __forceinline__ void lane_blocks(Ctx& t, const Outputs& o, uint32_t c
             }
         }
         __syncwarp();
+        if (!fits) {
+            lc.cur = kNoPos;
+            lc.direct = 0;
+            // (pending children that another warp left are used up first)
+            if (lane == 0) t.arena[cur + F_FLAGS] |= again ? FL_BUILD : s ? FL_ONE1 : FL_ONE0;
+            __syncwarp();
+            return false;
+        }
     }
     const uint32_t own = sh.own, opp = sh.opp, sat0 = sh.sat0, ss = sh.ss, z0 = sh.z0;
     const uint32_t nws = sh.nws, nwo = sh.nwo;
@@ -281,10 +291,6 @@ __device__ __forceinline__ void lane_blocks(Ctx& t, const Outputs& o, uint32_t c
         const bool live = (todo >> lane) & 1u;
         pbase = pos;
         if (!again) pos += nc;
-        if (!fits) {
-            pend = todo;
-            break;
-        }
         uint32_t coff = 0, cdeg = 0;
         // members that c misses
         uint32_t mc = 0;
@@ -559,10 +565,11 @@ __device__ __forceinline__ void lane_blocks(Ctx& t, const Outputs& o, uint32_t c
         f[F_FLAGS] = pend && !direct ? f[F_FLAGS] | FL_BUILD : f[F_FLAGS] & ~FL_BUILD;
     }
     __syncwarp();
-    lc.cur = fits ? cur : kNoPos;
+    lc.cur = cur;
     lc.next = again ? kNoPos : pos;
     lc.direct = direct;
     *nodes = done;
+    return true;
 }
 
 // Collects the universe of the pending child `bit` of the last block's frame (h:

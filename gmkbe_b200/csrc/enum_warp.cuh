@@ -49,6 +49,13 @@ constexpr uint32_t FL_SHARED1 = 512u;     //   parent's list, read in place (not
                                           //   the frame)
 constexpr uint32_t FL_BUILD = 1024u;      // frame flag: the pending children of its global side
                                           //   are built (they do not fit lane_blocks)
+// Frame flags: lane_blocks has nothing to decide the children of U / V with (no
+// member bounds them, or its row or list is too long): they are built one by one.
+// Members or k past kLaneMembers / kLaneK say the same without a flag.  A hub with
+// 200 leaves, whose frames all are like that: 83 ms when each block asked again, 70
+// here, 77 before there were blocks; four hubs of 60 47, 38 and 42.
+constexpr uint32_t FL_ONE0 = 2048u, FL_ONE1 = 4096u;
+constexpr uint32_t kLaneMembers = 15, kLaneK = 9;
 constexpr uint32_t kBitsMinList = 64;     // default: shorter lists filter their children by
                                           //   probing (gmk_opts.bits_min_list)
 constexpr uint32_t kBitsMaxZ = 8;         // bitmaps for at most this many members
@@ -1364,6 +1371,11 @@ __device__ int enter_node(Ctx& t, const Outputs& o, uint32_t cur, ChildReq* req,
 
 enum : int { NEXT_NONE = 0, NEXT_CHILD = 1, NEXT_BLOCK = 2 };
 
+// Are the children of side s (global) of a frame built one by one?
+__device__ __forceinline__ bool one_by_one(const Ctx& t, uint32_t flags, uint32_t ns, int s) {
+    return (flags & (s ? FL_ONE1 : FL_ONE0)) || ns > kLaneMembers || t.k > kLaneK;
+}
+
 // Warp form of next_child (enum_core.cuh): advances frame cur to its next
 // child and describes it in *req.  The children of a global side are first
 // looked at in blocks (lane_blocks): NEXT_BLOCK says that one is due (*hdr the
@@ -1393,8 +1405,9 @@ __device__ int next_child(Ctx& t, uint32_t cur, bool blocks, ChildReq* req, Hdr*
                 if (t.lane == 0) f[F_CNT0 + s] = pend & (pend - 1);
                 have = NEXT_CHILD;
             } else if (pos < end) {
-                if (!blocks) { c = pos; ++pos; }
-                have = blocks ? NEXT_BLOCK : NEXT_CHILD;
+                const bool one = !blocks || one_by_one(t, h.flags, h.ns, s);
+                if (one) { c = pos; ++pos; }
+                have = one ? NEXT_CHILD : NEXT_BLOCK;
             }
         } else if (pos < (h.end < h.cnt.get(s) ? h.end : h.cnt.get(s))) {
             p = pos;
@@ -1526,18 +1539,21 @@ __device__ bool split_path(Ctx& t, const SplitBuf& sb, uint32_t cur) {
 // pending children, and whether a second phase follows.
 struct Rest {
     uint32_t pos, lim, pend;
-    bool by_block;      // a global side: its range is handed out in blocks of 32
+    bool global;        // a global side: long ranges are handed out in blocks of 32
+    bool by_block;      // one that lane_blocks decides: short ones are not
     bool next_phase;
     // anything to hand out?  (a range of one block stays; the second phase goes
     // only when the first is used up)
     __device__ __forceinline__ bool range() const { return lim - pos > (by_block ? 32u : 0u); }
+    __device__ __forceinline__ uint32_t unit() const { return by_block || (global && lim - pos > 32) ? 32u : 1u; }
     __device__ __forceinline__ bool any() const {
         return range() || pend || (lim == pos && next_phase);
     }
 };
 
-__device__ __forceinline__ Rest frame_rest(const GraphView& g, const uint32_t* f) {
-    Rest r{0, 0, 0, false, false};
+__device__ __forceinline__ Rest frame_rest(const Ctx& t, const uint32_t* f) {
+    const GraphView& g = t.g;
+    Rest r{0, 0, 0, false, false, false};
     const uint32_t phase = f[F_PHASE];
     if (phase >= 2) return r;
     const uint32_t order = f[F_ORDER];
@@ -1548,7 +1564,8 @@ __device__ __forceinline__ Rest frame_rest(const GraphView& g, const uint32_t* f
     r.pos = f[F_POS];
     r.lim = f[F_END] < side ? f[F_END] : side;
     if (r.pos > r.lim) r.pos = r.lim;
-    r.by_block = global;
+    r.global = global;
+    r.by_block = global && !one_by_one(t, flags, f[F_NS], s);
     r.pend = global ? f[F_CNT0 + s] : 0u;
     if (phase == 0 && !(flags & FL_ONE_PHASE)) {
         const int s2 = 1 - s;
@@ -1573,12 +1590,12 @@ constexpr uint32_t kMaxDonateParts = GMK_DONATE_PARTS;
 __device__ __forceinline__ bool donate_top(Ctx& t, const Donation& db, uint32_t cur,
                                            unsigned long long want) {
     uint32_t best = kNoPos;
-    Rest rb{0, 0, 0, false, false};
+    Rest rb{0, 0, 0, false, false, false};
     #pragma unroll 1
     for (uint32_t x = cur; x != kNoPos; x = t.arena[x + F_PARENT_SLOT]) {
         const uint32_t* f = t.arena + x;
         if (!(f[F_FLAGS] & FL_ENTERED)) continue;
-        const Rest r = frame_rest(t.g, f);
+        const Rest r = frame_rest(t, f);
         if (r.any()) { best = x; rb = r; }
     }
     if (best == kNoPos) return false;
@@ -1592,9 +1609,11 @@ __device__ __forceinline__ bool donate_top(Ctx& t, const Donation& db, uint32_t 
     // warps waiting, up to kMaxDonateParts records of equal shares), the
     // donor keeps the rest
     // (a global side's range is split in blocks of 32 children, which cost
-    // lane_blocks as much as one; the children it left pending by their mask)
+    // lane_blocks as much as one, and single ones keep hubs busy with records: 73 ms
+    // in place of 70 for one of 200 leaves; the children it left pending by their
+    // mask)
     const bool by_range = rb.range(), by_mask = !by_range && rb.pend != 0;
-    const uint32_t unit = rb.by_block ? 32u : 1u;
+    const uint32_t unit = rb.unit();
     const uint32_t rem = by_range ? (rb.lim - rb.pos + unit - 1) / unit : by_mask ? __popc(rb.pend) : 0u;
     uint32_t parts = 1;
     if (rem >= 3 && want > 1) {
@@ -1875,10 +1894,9 @@ __device__ __forceinline__ unsigned long long run_dfs(Ctx& t, const Outputs& o, 
                     if (nx == NEXT_NONE) { cur = f[F_PARENT_SLOT]; continue; }
                     if (nx == NEXT_BLOCK) {
                         uint32_t n = 0;
-                        lane_blocks<kRec>(t, o, cur, h, req.s, req.opp_done, lc, &n);
+                        if (lane_blocks<kRec>(t, o, cur, h, req.s, req.opp_done, lc, &n)) polls = 8;
                         t.nodes += n;
                         task_nodes += n;
-                        polls = 8;
                         continue;
                     }
                 }
@@ -1899,7 +1917,7 @@ __device__ __forceinline__ unsigned long long run_dfs(Ctx& t, const Outputs& o, 
                 if (t.lane == 0) {
                     const int s = fa[F_PHASE] == 0 ? (int)fa[F_ORDER] : 1 - (int)fa[F_ORDER];
                     if (reenter) fa[F_FLAGS] &= ~FL_ENTERED;
-                    else if (lim.blocks && (fa[F_FLAGS] & gbit(s))) fa[F_CNT0 + s] |= 1u << (t.src[kSrcCap + 2] - fa[F_OFF0 + s]);
+                    else if (lim.blocks && (fa[F_FLAGS] & gbit(s)) && !one_by_one(t, fa[F_FLAGS], fa[F_NS], s)) fa[F_CNT0 + s] |= 1u << (t.src[kSrcCap + 2] - fa[F_OFF0 + s]);
                     else fa[F_POS] -= 1;
                 }
                 __syncwarp();
