@@ -29,7 +29,8 @@ EXPORTS = ("gmk_graph_load", "gmk_graph_from_csr", "gmk_graph_info", "gmk_graph_
            "gmk_abi_version", "gmk_root_features", "gmk_mlp_create", "gmk_mlp_free",
            "gmk_mlp_params", "gmk_mlp_gradient", "gmk_mlp_train", "gmk_mlp_predict",
            "gmk_mlp_predict_roots",
-           "gmk_root_costs", "gmk_plan_tasks", "gmk_graph_set_hash_load")
+           "gmk_root_costs", "gmk_plan_tasks", "gmk_graph_set_hash_load",
+           "gmk_collect", "gmk_collect_free")
 
 SCHEDULES = {"plain": 0, "batched": 1, "ordered": 2}
 ENGINES = {"warp": 0, "thread": 1}
@@ -76,7 +77,7 @@ class _Task(ctypes.Structure):
                 ("graph", ctypes.c_uint32), ("cost", ctypes.c_float)]
 
 
-class _Collector(ctypes.Structure):
+class _Collector(ctypes.Structure):      # gmk_collector
     _fields_ = [("data", ctypes.c_void_p), ("len", ctypes.c_uint64), ("cap", ctypes.c_uint64),
                 ("failed", ctypes.c_int32)]
 

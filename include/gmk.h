@@ -183,6 +183,20 @@ typedef struct {
 typedef int (*gmk_sink)(void* user, const uint32_t* x, uint32_t nx, const uint32_t* y,
                         uint32_t ny);
 
+/* A sink of the library's own, for callers that take all records together (a
+ * binding, for which a call back per record is dear): gmk_collect, with a
+ * gmk_collector as `user`, appends each record as nx, ny, x..., y... to data.
+ * Start from a zeroed gmk_collector; set len to 0 to use it again; gmk_collect_free
+ * releases data and zeroes it.  When memory runs out `failed` is set and the run is
+ * stopped (GMK_E_SINK). */
+typedef struct {
+    uint32_t* data;
+    uint64_t len, cap;        /* words used and allocated */
+    int32_t failed;
+} gmk_collector;
+int gmk_collect(void* user, const uint32_t* x, uint32_t nx, const uint32_t* y, uint32_t ny);
+void gmk_collect_free(void* user);
+
 /* Fills *o with the defaults: k = 1 as the reference's -k (src/main.cu:1722-1732),
  * no result limit (the gmk CLI applies the reference's -r default of 10^7), the
  * batched schedule and the warp engine. */
