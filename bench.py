@@ -22,7 +22,12 @@ build, root features, model prediction, planning, enumeration and read-back
 all inside the timed region.  L2 is flushed (256 MB write) between steps.
 
 Beside it: the plain schedule (one task per root, id order, no splitting) and
-the batched schedule without the model on the same graph; cl20k's throughput
+the batched schedule without the model on the same graph.  Graphs with a side
+above 128 take the list-based kernel, where the plain schedule also builds every
+child by itself; `plain_same_kernel` is one task per root, id order, no splitting
+with the children decided in lane blocks as the other schedules do it, so
+`learned_vs_plain_same_kernel` is what scheduling alone is worth and
+`learned_vs_plain` holds both.  Further: cl20k's throughput
 run (full graph, first 10^6 results) and the Chung-Lu 100k x 300k (cl100k) and
 500k x 1M (cl500k) graphs (first 10^7 / 10^8 results) under the three
 schedules; and complete enumerations of the Erdos-Renyi 200 x 200 graph (er200)
@@ -230,14 +235,24 @@ def _model(device: int):
     return L.load_default(device, os.path.join(ROOT, "_graphs", "subtree.npy")), "trained at start"
 
 
+# one task per root in id order, never split or shared: the plain schedule with
+# the batched schedules' kernel
+STATIC = dict(schedule="batched", chunk=0xFFFFFFFF, sharing=False, split_min_nodes=0xFFFFFFFF)
+
+
 def _schedules(g, k, limit, cost, reps, flush, check=None, **kw):
     """plain / batched / learned device times of one (graph, k, limit): the
     median of `reps` runs after one untimed run each; sets compared."""
     import torch
     out, summ = {}, {}
     import gmkbe_b200 as G
-    for name, extra in (("learned", dict(schedule="ordered", task_cost=cost)),
-                        ("batched", dict(schedule="batched")), ("plain", dict(schedule="plain"))):
+    arms = [("learned", dict(schedule="ordered", task_cost=cost)), ("batched", dict(schedule="batched")),
+            ("plain", dict(schedule="plain"))]
+    if max(g.n_left, g.n - g.n_left) > 128:      # (smaller ones: plain is on the same kernel)
+        # (a shard's tasks are planned by cost, whole roots for plain only)
+        if not kw.get("nshards"):
+            arms.append(("plain_same_kernel", STATIC))
+    for name, extra in arms:
         try:
             g.enumerate(k=k, result_limit=limit, **extra, **kw)
             ms, st = [], None
@@ -253,9 +268,11 @@ def _schedules(g, k, limit, cost, reps, flush, check=None, **kw):
         out[name] = {"ms": m, "results": st.count, "value": st.count / (m / 1e3),
                      "rounds": st.rounds, "donations": st.donations, "tasks": st.tasks}
         summ[name] = st.summary()
-    if any("error" in out[n] for n in ("learned", "batched", "plain")):
+    if any("error" in out[n] for n, _ in arms):
         return out
     out["learned_vs_plain"] = out["plain"]["ms"] / out["learned"]["ms"]
+    if "plain_same_kernel" in out:
+        out["learned_vs_plain_same_kernel"] = out["plain_same_kernel"]["ms"] / out["learned"]["ms"]
     out["batched_vs_plain"] = out["plain"]["ms"] / out["batched"]["ms"]
     out["learned_vs_batched"] = out["batched"]["ms"] / out["learned"]["ms"]
     if not limit:
@@ -412,6 +429,8 @@ def run_gmk(args, world, rank, local):
                     "d2h_bytes_per_step": d2h},
             "gpu_launches": launches,
             "learned_vs_plain": sched.get("learned_vs_plain"),
+            # scheduling alone (learned_vs_plain also holds plain's own, child by child node kernel)
+            "learned_vs_plain_same_kernel": sched.get("learned_vs_plain_same_kernel"),
             "schedules": sched,
             "roofline": {
                 "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
