@@ -158,6 +158,8 @@ struct Outputs {
                                     //   (null: the limit raises `stop`)
 };
 
+static constexpr uint32_t kSatCap = 16;   // k <= 15, and k + 1 sources fit kSatCap + 1
+
 struct Task {
     GraphView g;
     uint32_t k;
@@ -252,7 +254,7 @@ GMK_HD bool outsider_addable(Task& t, const uint32_t* l0, uint32_t n0, const uin
             if (tots[o][i] >= t.k && degree(g, lst[o][2 * i]) < hard_deg) {
                 hard = lst[o][2 * i]; hard_deg = degree(g, hard);
             }
-        uint32_t src[4];
+        uint32_t src[kSatCap + 1];
         uint32_t nsrc = 0;
         if (hard != 0xFFFFFFFFu) {
             src[nsrc++] = hard;
@@ -340,7 +342,7 @@ GMK_HD bool outsider_addable_mixed(Task& t, int s, uint32_t lo, const uint32_t* 
         if (tot[q] >= t.k && degree(g, w) < hard_deg) { hard = w; hard_deg = degree(g, w); }
     }
     const uint32_t nopp = nm + n;
-    uint32_t src[17];
+    uint32_t src[kSatCap + 1];
     uint32_t nsrc = 0;
     if (hard != 0xFFFFFFFFu) {
         src[nsrc++] = hard;
@@ -485,7 +487,6 @@ GMK_HD void normalise(const GraphView& g, uint32_t* f) {
 
 enum : int { ENTER_ITERATE = 0, ENTER_DONE = 1, ENTER_PUSHED = 2 };
 static constexpr uint32_t kNoPos = 0xFFFFFFFFu;
-static constexpr uint32_t kSatCap = 16;   // k <= 16
 
 // Build the child "S + c" of frame `cur` at the arena top.  c is on side s,
 // at local position p (kNoPos for a global side).  `forced`: every other
