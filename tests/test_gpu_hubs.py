@@ -21,6 +21,7 @@ GRAPHS = {
     "star_u": (lambda: _star(140, True), 1),
     "star_k2": (lambda: _star(135, False), 2),
     "two_hubs": (lambda: gg.hubs_and_sparse(2, 70, 140, 2, 3), 1),
+    "three_hubs": (lambda: gg.hubs_and_sparse(3, 31, 145, 2, 7), 1),
 }
 
 
