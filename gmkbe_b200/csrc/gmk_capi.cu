@@ -1258,9 +1258,12 @@ std::vector<uint32_t> select_roots(uint32_t nl, const float* cost, uint32_t rb, 
 
 // Narrowest chunk of first-level children: of gmk_plan_tasks and of the thread
 // engine's tasks, and of the tasks that a run of the list-based kernel makes itself
-// -- that one looks at its children 32 at a time.  (The thread engine never
-// splits a task, so its tail is its widest one: er200, k = 1 takes 1.60 s with 16
-// and 3.95 s with 64.)
+// -- that one looks at its children 32 at a time -- where warps share inside the
+// launch.  A run that does not share (records, no_sharing) keeps narrow ones: its
+// first launch has no more parallelism than tasks (117 x 80, k = 2, the first
+// 20 000 records: 0.14 ms with 16, 0.64 with 64; 168 x 39 with hubs, k = 1, counted
+// without sharing: 5.9 and 9.3).  The thread engine never splits a task, so its tail is
+// its widest one: er200, k = 1 takes 1.60 s with 16 and 3.95 s with 64.
 constexpr uint32_t kPlanChunk = 16;
 constexpr uint32_t kMinChunk = 64;
 
@@ -1729,7 +1732,13 @@ int run_jobs(std::vector<GraphJob>& jobs, const gmk_opts* opts, gmk_sink sink, v
     const bool planned = is_planned(jobs, opts);
     std::vector<gmk_task> plan;
     const uint32_t max_chunks = opts->schedule == GMK_SCHEDULE_PLAIN ? 1u : 0xFFFFFFFFu;
-    const uint32_t min_chunk = warp ? kMinChunk : kPlanChunk;
+    // the warp engine splits unfinished trees (batched / ordered schedules) ...
+    const uint32_t split_min = (!warp || opts->schedule == GMK_SCHEDULE_PLAIN)
+                                   ? 0u
+                                   : (opts->split_min_nodes ? opts->split_min_nodes : 64u);
+    // ... and shares them inside a launch in count-only runs
+    const bool share = warp && split_min && !opts->emit && !opts->no_sharing;
+    const uint32_t min_chunk = share ? kMinChunk : kPlanChunk;
     if (planned && (rc = plan_jobs(jobs, opts, di.sms, workers, max_chunks, min_chunk, plan))) return rc;
     unsigned long long n_tasks = 0;
     for (size_t i = 0; i < ng; ++i) {
@@ -1793,10 +1802,6 @@ int run_jobs(std::vector<GraphJob>& jobs, const gmk_opts* opts, gmk_sink sink, v
         if ((rc = grow((void**)&ws.d_out, &ws.out_bytes, out_words * 4ull * (warp ? 2 : 1))))
             return rc;
     }
-    // the warp engine splits unfinished trees (batched / ordered schedules)
-    const uint32_t split_min = (!warp || opts->schedule == GMK_SCHEDULE_PLAIN)
-                                   ? 0u
-                                   : (opts->split_min_nodes ? opts->split_min_nodes : 64u);
     unsigned long long split_word_cap = 0, split_idx_cap = 0;
     if (warp) {   // split records: load balance, record-buffer draining, and round bookkeeping
         split_word_cap = std::max<unsigned long long>(1ull << 22, workers * 8192ull);
@@ -1808,8 +1813,7 @@ int run_jobs(std::vector<GraphJob>& jobs, const gmk_opts* opts, gmk_sink sink, v
                 return rc;
         }
     }
-    // in-launch work sharing (count-only warp runs that split: batched / ordered)
-    const bool share = warp && split_min && !opts->emit && !opts->no_sharing;
+    // in-launch work sharing
     unsigned long long dq_word_cap = 0, dq_idx_cap = 0;
     if (share) {
         dq_word_cap = std::max<unsigned long long>(1ull << 22, workers * 4096ull);

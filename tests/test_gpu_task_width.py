@@ -1,6 +1,8 @@
 """How wide the tasks are that a run makes itself.  The thread engine takes a
 task's children one after the other and never splits it, so it keeps narrow
-ones (16 first-level children) on every schedule."""
+ones (16 first-level children) on every schedule; so do runs of the warp engine
+that do not share inside a launch: their first launch has no more parallelism than
+tasks."""
 import pytest
 
 import gmkbe_b200 as G
@@ -28,3 +30,19 @@ def test_thread_engine_tasks_are_sixteen_children_wide(golden, name):
         assert st.summary() == want
         m = max(1, nv // 16)
         assert st.tasks == h.n_left * -(-nv // -(-nv // m))
+
+
+@pytest.mark.parametrize("kw", [dict(collect=True), dict(sharing=False)])
+def test_tasks_of_runs_without_sharing_are_sixteen_children_wide(kw):
+    g = gg.erdos_renyi(60, 150, 0.02, 5)
+    nv = g.n - g.n_left
+    with G.Graph.from_graph(g) as dg:
+        want = dg.enumerate(k=1).summary()
+        # (nothing is split, so the tasks are the first launch's)
+        st = dg.enumerate(k=1, split_min_nodes=0xFFFFFFFF, **kw)
+        assert st.summary() == want and st.rounds == 1
+        assert st.tasks == g.n_left * -(-nv // 16)
+        st = dg.enumerate(k=1, split_min_nodes=0xFFFFFFFF, schedule="ordered", task_cost=dg.root_costs(),
+                          tasks_per_worker=1 << 20, **kw)
+        assert st.summary() == want and st.rounds == 1
+        assert st.tasks == g.n_left * -(-nv // -(-nv // (nv // 16)))
