@@ -37,7 +37,14 @@ namespace gmk {
 namespace warp {
 
 constexpr uint32_t kBitsSide = 32;       // universe vertices per side: one per lane
-constexpr uint32_t kBitsScanMax = 2048;  // outsider source-row entries in total
+constexpr uint32_t kBitsScanMax = 2048;  // a lane block child: entries of the row that bounds the other side
+// Entries of the rows that bound one side's outsiders at a node that the list-based
+// search hands over.  Below a hub they number hundreds, each with its probes, for
+// subtrees of a node or two, where the list-based rules stop at the first vertex that
+// can join: 168 x 39 with hubs of 168, k = 1, counted without sharing 6.0 ms with rows
+// up to 2 048, 4.6 with 160 (and with 64); er200 and the Chung-Lu prefixes have shorter
+// ones.
+constexpr uint32_t kBitsRow = 160;
 constexpr uint32_t kBitsSubset = 5;   // 2^5 subsets: one per lane
 constexpr uint32_t kBitsStack = 64;      // one entry per included candidate, at most
 constexpr uint32_t kBitsBudget = 8;   // nodes between two polls of the search loop
@@ -113,7 +120,7 @@ __device__ __forceinline__ bool bits_source(const Ctx& t, BitSources& src, int s
         }
         if (sum < cost) { pick = pk; cost = sum; }
     }
-    if (cost > kBitsScanMax) return false;
+    if (cost > kBitsRow) return false;
     #pragma unroll 1
     for (; pick; pick &= pick - 1) {
         const uint32_t i = __ffs(pick) - 1;
