@@ -29,8 +29,8 @@
 // instructions for 1.83 M results, most of them setting universes up).  A node of
 // the list-based search costs 1 000-1 600 warp instructions, hash probes and list
 // traffic, one on masks 100-400.  Measured with lane blocks and the wider
-// register allocation (ms, complete runs, one B200): er200 k = 1 27.0 -> 10.9, 400 x
-// 400 degree 5 19.6 -> 6.4, 200 x 200 degree 5, k = 2, first 3 10^6 28.0 -> 6.9.
+// register allocation (ms, complete runs, one B200): er200 k = 1 27.6 -> 11.5, 400 x
+// 400 degree 5 19.7 -> 6.6, 200 x 200 degree 5, k = 2, first 3 10^6 28.0 -> 6.9.
 #pragma once
 
 namespace gmk {

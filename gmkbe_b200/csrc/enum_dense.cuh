@@ -39,8 +39,8 @@
 // lists, and their L2 latency; this one spent 640 with N = 3 masks (77 x 77, k
 // = 2, before the fans: 10.3 G instructions for 12.4 M results, 43 % of the
 // issue slots active) and nothing leaves the SM.  Measured, complete runs, list-based -> here (ms,
-// one B200): 18 x 14 k = 1 0.90 -> 0.13, k = 3 19.5 -> 0.29; 58 x 58 k = 2 30.3 ->
-// 2.35; 77 x 77 k = 2 115 -> 10.6; 82 x 83 k = 2 31.6 -> 8.5; 128 x 128 k = 1
+// one B200): 18 x 14 k = 1 0.90 -> 0.12, k = 3 19.5 -> 0.29; 58 x 58 k = 2 30.3 ->
+// 2.4; 77 x 77 k = 2 115 -> 10.6; 82 x 83 k = 2 31.6 -> 8.5; 128 x 128 k = 1
 // 10.4 -> 2.2.
 #pragma once
 #include "enum_warp.cuh"
@@ -395,9 +395,10 @@ __device__ __forceinline__ bool pop(Ctx<N>& t, State<N>& s) {
     return true;
 }
 
-// One node: prunes, takes results, or goes on to another state (true): the child
-// that includes the branching candidate (the state that excludes it is pushed),
-// or, after a fan whose children are all done, the state without them.
+// One node: prunes, takes results, or goes on (true) to the child that includes the
+// branching candidate, to be refitted; the state that excludes it is pushed.  A fan is
+// pushed as one entry (false): pop hands out its children, to be refitted too, and
+// then the state without them.
 template <int N>
 __device__ __forceinline__ bool node(Ctx<N>& t, State<N>& s, bool fit) {
     if (kFans<N> && fit) refit<N>(t, s);

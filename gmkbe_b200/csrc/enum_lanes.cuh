@@ -28,7 +28,8 @@
 // or a longer row, go to the bit-mask search straight from here (lane_child):
 // their universe comes from the same lists and rows, so no frame is built.  The
 // rest (a side stays global, c adjacent to z0, a side of more than 32 vertices)
-// is built the usual way.  Both kinds are left pending in the frame, as a mask
+// is built the usual way, and so are all children of a frame that has no z0, too
+// long a row or list, or more than 15 members (FL_ONE0, FL_ONE1).  Both kinds are left pending in the frame, as a mask
 // in the words of the list that a global side does not have.  Where a child
 // goes depends on the frame and the child alone, so the tree does not depend on
 // how its range was cut.

@@ -52,8 +52,8 @@ constexpr uint32_t FL_BUILD = 1024u;      // frame flag: the pending children of
 // Frame flags: lane_blocks has nothing to decide the children of U / V with (no
 // member bounds them, or its row or list is too long): they are built one by one.
 // Members or k past kLaneMembers / kLaneK say the same without a flag.  A hub with
-// 200 leaves, whose frames all are like that: 83 ms when each block asked again, 70
-// here, 77 before there were blocks; four hubs of 60 47, 38 and 42.
+// 200 leaves, whose frames all are like that: 84 ms when each block asked again, 73
+// here, 78 before there were blocks; four hubs of 60 47, 39 and 42.
 constexpr uint32_t FL_ONE0 = 2048u, FL_ONE1 = 4096u;
 constexpr uint32_t kLaneMembers = 15, kLaneK = 9;
 constexpr uint32_t kBitsMinList = 64;     // default: shorter lists filter their children by
@@ -1615,9 +1615,8 @@ __device__ __forceinline__ bool donate_top(Ctx& t, const Donation& db, uint32_t 
     // warps waiting, up to kMaxDonateParts records of equal shares), the
     // donor keeps the rest
     // (a global side's range is split in blocks of 32 children, which cost
-    // lane_blocks as much as one, and single ones keep hubs busy with records: 73 ms
-    // in place of 70 for one of 200 leaves; the children it left pending by their
-    // mask)
+    // lane_blocks as much as one; a hub's single children, each a record, cost one
+    // of 200 leaves 4 %; the children it left pending by their mask)
     const bool by_range = rb.range(), by_mask = !by_range && rb.pend != 0;
     const uint32_t unit = rb.unit();
     const uint32_t rem = by_range ? (rb.lim - rb.pos + unit - 1) / unit : by_mask ? __popc(rb.pend) : 0u;

@@ -152,9 +152,12 @@ constexpr int kWarpsPerBlock = kWBlock / 32;
 // instruction-cache misses (28 warps at 72 registers: an issue slot in five
 // used, 19 of 36 stall cycles for instructions): 12 warps at 168 registers,
 // without spills, are faster almost everywhere (er200 k = 1 14.6 -> 10.9 ms, cl20k
-// first million 0.40 -> 0.23, cl100k k = 2 10.0 -> 7.7, cl500k k = 2 48.1 -> 41.6).
-// The exception is k = 1 over an edge hash far larger than L2 (cl500k, 537 MB),
-// whose probes wait for HBM: 28 warps 7.9 ms, 12 warps 10.0.
+// first million 0.40 -> 0.23; before long loops looked at the stop flag, cl100k k = 2
+// 10.0 -> 7.7 and cl500k k = 2 48.1 -> 41.6).
+// The exception is k = 1 over an edge hash larger than L2, whose probes wait for HBM.
+// First 10^8 results of Chung-Lu graphs, 28 and 12 warps (ms): hash of 16 MB 31.1 and
+// 26.9, 134 MB 6.6 and 7.0 (2.7 M edges) or 6.5 and 9.0 (3.2 M), 268 MB 6.6 and 9.1, 537 MB
+// 6.9 and 9.4.  The line is at the upper end of that: 134 and 268 MB would gain as well.
 constexpr int kWarpMinBlocks = 10;
 constexpr int kManyMinBlocks = 25;
 constexpr size_t kManyHashBytes = 256ull << 20;

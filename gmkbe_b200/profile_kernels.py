@@ -6,9 +6,9 @@
 In launch order: csr_check_kernel and build_edge_hash (loading the graph),
 root_cost_kernel (gmk_root_costs), root_features_kernel (gmk_root_features),
 float_to_half_kernel + forward_kernel (a prediction over every root),
-float_to_half_kernel, forward_kernel, backward_kernel, adam_kernel (one
-training epoch over `samples` feature rows), forward_kernel + backward_kernel
-again (the loss after the epoch), and the enumeration (enumerate_warp_kernel,
+float_to_half_kernel, gradient_kernel, gradient_sum_kernel, adam_kernel (one
+training epoch over `samples` feature rows), the two gradient kernels again
+(the loss after the epoch), and the enumeration (enumerate_warp_kernel,
 result limit `limit`).  Prints the times the API reports.  Under ncu, select
 kernels with -k and count launches with -c.
 """

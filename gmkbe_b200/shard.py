@@ -1,5 +1,6 @@
 """Multi-GPU runs: one process per GPU, each enumerating its shard of the
-search tasks (gmk_opts.shard / nshards: task t goes to rank t % world).
+search tasks (gmk_opts.shard / nshards: the longest-processing-time partition
+of the planned tasks).
 
 The shards share nothing while they run.  At the end the per-rank set
 summaries are combined once: counts and h1 sums add (mod 2^64), h2 values

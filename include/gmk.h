@@ -80,8 +80,8 @@ void gmk_graph_free(gmk_graph* g);
  * first-level children). */
 enum {
     GMK_SCHEDULE_PLAIN = 0,    /* one task per root, roots in id order (largest task_cost
-                                  first when one is given), no splitting,
-                                  children built one by one */
+                                  first when one is given), no splitting; the list-based
+                                  search then builds children one by one */
     GMK_SCHEDULE_BATCHED = 1,  /* roots split into chunks, persistent work queue; unfinished
                                   search trees are split into the next round's tasks */
     GMK_SCHEDULE_ORDERED = 2   /* batched over planned tasks: roots split into chunks in
