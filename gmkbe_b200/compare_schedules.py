@@ -7,7 +7,9 @@ Full enumeration is where scheduling matters: with a result limit every warp
 stays busy until the limit, but a complete run ends with the last, largest
 search tree.  Each case reports device time (CUDA events) per schedule and
 checks that every schedule gives the same set summary.
-  * plain   -- one task per root in id order, no splitting;
+  * plain   -- one task per root in id order, no splitting; above 128 vertices a
+               side also with children built one by one, where the others
+               decide them in lane blocks (a ratio against it holds both);
   * batched -- roots cut into chunks, chunk-major queue, unfinished trees
                split into the next round;
   * learned -- batched, roots ordered by the subtree-size model's predicted
